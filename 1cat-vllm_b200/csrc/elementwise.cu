@@ -126,6 +126,118 @@ __global__ void silu_and_mul_kernel(const __nv_bfloat16* __restrict__ x, __nv_bf
   *reinterpret_cast<uint4*>(y + t * I + c) = o;
 }
 
+// The same in 16-byte accesses: a group of D / 8 lanes owns a head, a lane eight neighbouring elements of it; the other element of each rotary
+// pair comes from the lane half a rotary width away. A group takes HU heads of a token with their loads in flight together and the token's
+// cosines and sines read once. Bound by memory: a prompt's q, k and v once in and once out. Two-byte accesses with a warp per head
+// (rope_cache_kernel below) reached 0.8 TB/s at 8192 tokens x 56 heads of 128 (295 us); this one
+// takes 80 us (2.9 TB/s); at 64 tokens 8 us for 10.
+template <int D, int HU>
+__global__ void __launch_bounds__(256) rope_cache_vec_kernel(const RopeCacheParams p) {
+  constexpr int LPH = D / 8;                     // lanes of a head
+  pdl_trigger();
+  pdl_wait();
+  const int heads = p.Hq + 2 * p.Hkv, per_tok = (heads + HU - 1) / HU;
+  const int unit = blockIdx.x * (256 / LPH) + threadIdx.x / LPH;
+  const int t = unit / per_tok, h0 = (unit - t * per_tok) * HU;
+  const int lane = threadIdx.x & 31, sub = threadIdx.x % LPH, i0 = sub * 8;
+  const bool live = t < p.T;                     // every lane stays for the shuffles
+  __nv_bfloat16* src[HU];
+  uint4 raw[HU];
+#pragma unroll
+  for (int u = 0; u < HU; ++u) {
+    const int hh = h0 + u;
+    src[u] = nullptr;
+    raw[u] = make_uint4(0, 0, 0, 0);
+    if (live && hh < heads) {
+      if (hh < p.Hq) src[u] = p.q + (size_t)t * p.q_st + (size_t)hh * p.q_sh;
+      else if (hh < p.Hq + p.Hkv) src[u] = p.k + (size_t)t * p.k_st + (size_t)(hh - p.Hq) * D;
+      else src[u] = p.v + (size_t)t * p.v_st + (size_t)(hh - p.Hq - p.Hkv) * D;
+      raw[u] = *reinterpret_cast<const uint4*>(src[u] + i0);
+    }
+  }
+  const int half = p.rot >> 1;
+  const bool first = i0 < half, rotates = i0 < p.rot;
+  const int f0 = first ? i0 : i0 - half;         // frequency of this lane's first element
+  const int partner = (lane & ~(LPH - 1)) + (rotates ? (first ? sub + (half >> 3) : sub - (half >> 3)) : sub);
+  __align__(16) float c[8], s[8];
+  if (live && rotates) {
+    const float* cs = p.cos_sin + (size_t)p.positions[t] * p.rot + f0;
+#pragma unroll
+    for (int i = 0; i < 8; i += 4) {
+      *reinterpret_cast<float4*>(c + i) = *reinterpret_cast<const float4*>(cs + i);
+      *reinterpret_cast<float4*>(s + i) = *reinterpret_cast<const float4*>(cs + half + i);
+    }
+  }
+  const int slot = live && p.kv_cache != nullptr ? p.slot_mapping[t] : -1;
+  const int page = slot >= 0 ? slot / p.bs : 0;
+  const size_t row0 = ((size_t)page * 2 * p.Hkv * p.bs + (size_t)(slot - page * p.bs)) * D + i0;   // key row of head 0; heads are bs rows apart
+#pragma unroll
+  for (int u = 0; u < HU; ++u) {
+    const int hh = h0 + u;
+    const int kind = hh < p.Hq ? 0 : (hh < p.Hq + p.Hkv ? 1 : 2);
+    const __nv_bfloat16* nw = kind == 0 ? p.q_norm : (kind == 1 ? p.k_norm : nullptr);
+    uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
+    float x[8];
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&w[i]));
+      x[2 * i] = f.x;
+      x[2 * i + 1] = f.y;
+      ss += f.x * f.x + f.y * f.y;
+    }
+#pragma unroll
+    for (int o = LPH / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (nw != nullptr) {
+      const float inv = rsqrtf(ss / (float)D + p.eps);
+      const uint4 gw = *reinterpret_cast<const uint4*>(nw + i0);
+      const uint32_t g4[4] = {gw.x, gw.y, gw.z, gw.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g4[i]));
+        // the normalised value is rounded to bf16 before the rotation, like the separate-kernel formulation
+        const __nv_bfloat162 b = __floats2bfloat162_rn(x[2 * i] * inv * (p.gemma ? 1.f + g.x : g.x), x[2 * i + 1] * inv * (p.gemma ? 1.f + g.y : g.y));
+        w[i] = *reinterpret_cast<const uint32_t*>(&b);
+        const float2 f = __bfloat1622float2(b);
+        x[2 * i] = f.x;
+        x[2 * i + 1] = f.y;
+      }
+    }
+    uint32_t pw[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) pw[i] = __shfl_sync(0xffffffffu, w[i], partner);
+    if (src[u] == nullptr) continue;
+    if (kind != 2) {
+      if (rotates) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 y = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&pw[i]));
+          const float a = first ? x[2 * i] * c[2 * i] - y.x * s[2 * i] : x[2 * i] * c[2 * i] + y.x * s[2 * i];
+          const float b = first ? x[2 * i + 1] * c[2 * i + 1] - y.y * s[2 * i + 1] : x[2 * i + 1] * c[2 * i + 1] + y.y * s[2 * i + 1];
+          const __nv_bfloat162 r = __floats2bfloat162_rn(a, b);
+          w[i] = *reinterpret_cast<const uint32_t*>(&r);
+        }
+      }
+      *reinterpret_cast<uint4*>(src[u] + i0) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    if (kind != 0 && slot >= 0) {
+      const size_t e = row0 + (size_t)(hh - p.Hq) * p.bs * D;   // value heads follow the key heads
+      if (p.kv_fp8) {
+        const float scale = kind == 1 ? p.k_scale_inv : p.v_scale_inv;
+        uint32_t b8[2] = {0, 0};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float2 f = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&w[i >> 1]));
+          b8[i >> 2] |= (uint32_t)(uint8_t)__nv_cvt_float_to_fp8(((i & 1) ? f.y : f.x) * scale, __NV_SATFINITE, __NV_E4M3) << ((i & 3) * 8);
+        }
+        *reinterpret_cast<uint2*>(reinterpret_cast<uint8_t*>(p.kv_cache) + e) = make_uint2(b8[0], b8[1]);
+      } else {
+        *reinterpret_cast<uint4*>(p.kv_cache + e) = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    }
+  }
+}
+
 // One warp per (token, head): optional RMSNorm over the head, NeoX rotary on the first `rot` dims (q and k, in place),
 // k and v rows copied into the paged cache [block][2][Hkv][bs][D] at slot_mapping[token].
 __global__ void rope_cache_kernel(RopeCacheParams p) {
@@ -294,6 +406,21 @@ int silu_and_mul_launch(const void* x, void* y, int T, int I, cudaStream_t st) {
 int rope_cache_launch(const RopeCacheParams& p, cudaStream_t st) {
   if (p.T == 0) return 0;
   if (p.D > 512 || p.rot > p.D || (p.rot & 1)) return -1;
+  // 16-byte accesses: heads of 64, 128 or 256 whose rotary halves are whole lanes, everything aligned, positions with one component
+  auto al = [](const void* x) { return ((uintptr_t)x & 15) == 0; };
+  if ((p.D == 64 || p.D == 128 || p.D == 256) && p.rot % 16 == 0 && p.mrope_s0 == 0 && al(p.q) && al(p.k) && al(p.v) && al(p.q_norm) && al(p.k_norm) &&
+      al(p.kv_cache) && (p.rot == 0 || al(p.cos_sin)) && p.q_st % 8 == 0 && p.q_sh % 8 == 0 && p.k_st % 8 == 0 && p.v_st % 8 == 0 &&
+      (long long)p.T * (p.Hq + 2 * p.Hkv) < (1LL << 30)) {
+    const int heads = p.Hq + 2 * p.Hkv, gpb = 256 / (p.D / 8);
+    // four heads per group once that still leaves several blocks for every SM; single heads when there are few tokens (shorter chains)
+    const bool four = (long long)p.T * ((heads + 3) / 4) >= 1024LL * gpb;
+    const long long units = (long long)p.T * (four ? (heads + 3) / 4 : heads);
+    const dim3 grid((unsigned)((units + gpb - 1) / gpb));
+    auto go = [&](auto kernel) { return launch_k(kernel, grid, dim3(256), 0, st, true, p) == cudaSuccess ? 0 : -2; };
+    if (p.D == 64) return four ? go(rope_cache_vec_kernel<64, 4>) : go(rope_cache_vec_kernel<64, 1>);
+    if (p.D == 128) return four ? go(rope_cache_vec_kernel<128, 4>) : go(rope_cache_vec_kernel<128, 1>);
+    return four ? go(rope_cache_vec_kernel<256, 4>) : go(rope_cache_vec_kernel<256, 1>);
+  }
   long long warps = (long long)p.T * (p.Hq + 2 * p.Hkv);
   int wpb = 8;
   launch_k(rope_cache_kernel, dim3((unsigned)((warps + wpb - 1) / wpb)), dim3(wpb * 32), wpb * p.D * sizeof(float), st, true, p);
