@@ -895,6 +895,7 @@ torch::Tensor mla_decode(torch::Tensor q_abs, torch::Tensor q_rope, torch::Tenso
   p.query_start_loc = qsl.data_ptr<int>(); p.seq_lens = seq_lens.data_ptr<int>(); p.block_table = block_table.data_ptr<int>();
   p.bt_stride = (int)block_table.stride(0); p.R = (int)seq_lens.size(0);
   p.bs = (int)cache.size(1); p.bs_shift = 0;
+  p.num_blocks = (int)cache.size(0);
   while ((1 << p.bs_shift) < p.bs) ++p.bs_shift;
   p.max_q_len = (int)max_q_len; p.splits = (int)splits; p.scale = (float)scale;
   check_sink_gate(sinks, gate, et, p.T, p.H);
@@ -910,6 +911,7 @@ torch::Tensor mla_decode(torch::Tensor q_abs, torch::Tensor q_rope, torch::Tenso
   return out;
 }
 
+bool mla_decode_wide(int64_t kv_lora) { return oc::mla_decode_tc_takes((int)kv_lora, 64, 16, 0, 1.f); }
 bool mla_tensor_core_sizes(int64_t kv_lora, int64_t rope_pad) { return oc::mla_tensor_core_sizes((int)kv_lora, (int)rope_pad); }
 
 // Expanded-form prefill, first half: the contexts of the listed requests gathered from their pages and the query rows in whole chunks.
@@ -1270,11 +1272,12 @@ void read_status_async(torch::Tensor pinned) {
   oc::mla_prefill_read_status_async(p + 10, st);
   oc::diff_prefill_read_status_async(p + 11, st);
   oc::talk_prefill_read_status_async(p + 12, st);
+  oc::mla_decode_tc_read_status_async(p + 13, st);
 }
 
 int64_t read_status(bool clear) {
   return (int64_t)(oc::gemm_read_status(clear) | oc::elementwise_read_status(clear) | oc::attention_read_status(clear) | oc::attention_tc_read_status(clear) |
-                   oc::comm_read_status(clear) | oc::gdn_read_status(clear) | oc::sampling_read_status(clear) | oc::moe_read_status(clear) | oc::mla_read_status(clear) | oc::mla_prefill_read_status(clear) | oc::diff_prefill_read_status(clear) | oc::talk_prefill_read_status(clear) | oc::ep_read_status(clear));
+                   oc::comm_read_status(clear) | oc::gdn_read_status(clear) | oc::sampling_read_status(clear) | oc::moe_read_status(clear) | oc::mla_read_status(clear) | oc::mla_decode_tc_read_status(clear) | oc::mla_prefill_read_status(clear) | oc::diff_prefill_read_status(clear) | oc::talk_prefill_read_status(clear) | oc::ep_read_status(clear));
 }
 
 // ---- symmetric slab + peer-memory reductions
@@ -1370,6 +1373,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("read_status_async", &read_status_async);
   m.def("mla_decode", &mla_decode);
   m.def("mla_tensor_core_sizes", &mla_tensor_core_sizes);
+  m.def("mla_decode_wide", &mla_decode_wide);
   m.def("mla_prepare", &mla_prepare);
   m.def("mla_prefill_inputs", &mla_prefill_inputs);
   m.def("mla_prefill", &mla_prefill);

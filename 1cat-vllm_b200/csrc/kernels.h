@@ -238,7 +238,12 @@ struct MlaParams {
   const float* sinks;           // [H] logits that join the softmax denominator only, or null
   const void* gate;             // [T][H] (row pitch gate_st): outputs are multiplied by its sigmoid, or null
   long long gate_st;
+  int num_blocks;               // pages of the cache
 };
+bool mla_decode_tc_takes(int kv_lora, int rope_pad, int bs, int fine, float scale);
+int mla_decode_tc_launch(const MlaParams& p, cudaStream_t st);
+unsigned int mla_decode_tc_read_status(bool clear);
+void mla_decode_tc_read_status_async(unsigned int* dst, cudaStream_t st);
 int mla_decode_launch(const MlaParams& p, cudaStream_t st);
 bool mla_tensor_core_sizes(int kv_lora, int rope_pad);
 // Prefill in the expanded form: gathered latents -> per-head keys and values (a GEMM in between) -> causal attention.

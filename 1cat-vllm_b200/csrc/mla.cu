@@ -270,14 +270,23 @@ __global__ void mla_combine_kernel(const MlaParams p) {
   const float L = warp_sum(lane < p.splits ? p.ws_ml[((size_t)lane * rows + warp) * 2 + 1] * f_mine : 0.f);
   const float den = L + (p.sinks != nullptr ? ex2(p.sinks[warp % p.H] * 1.4426950408889634f - M) : 0.f);
   const float inv = L > 0.f ? gate_of<__nv_bfloat16>(p, warp / p.H, warp % p.H) / den : 0.f;
-  for (int c = lane * 2; c < DV; c += 64) {
-    float x = 0.f, y = 0.f;
-    for (int s = 0; s < p.splits; ++s) {
-      const float f = __shfl_sync(0xffffffffu, f_mine, s);
-      const float2 v = *reinterpret_cast<const float2*>(p.ws_o + ((size_t)s * rows + warp) * DV + c);
-      if (f != 0.f) { x = fmaf(v.x, f, x); y = fmaf(v.y, f, y); }
+  // 16-byte loads, four splits of a column block in flight
+  for (int c = lane * 4; c < (DV + 127) / 128 * 128; c += 128) {
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s0 = 0; s0 < p.splits; s0 += 4) {
+      float4 v[4];
+      float f[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        f[i] = s0 + i < p.splits ? __shfl_sync(0xffffffffu, f_mine, s0 + i) : 0.f;
+        v[i] = f[i] != 0.f && c < DV ? *reinterpret_cast<const float4*>(p.ws_o + ((size_t)(s0 + i) * rows + warp) * DV + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (f[i] != 0.f) x = make_float4(fmaf(v[i].x, f[i], x.x), fmaf(v[i].y, f[i], x.y), fmaf(v[i].z, f[i], x.z), fmaf(v[i].w, f[i], x.w));
     }
-    *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)warp * DV + c) = pk(x * inv, y * inv);
+    if (c < DV)
+      *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)warp * DV + c) = make_uint2(pk(x.x * inv, x.y * inv), pk(x.z * inv, x.w * inv));
   }
 }
 
@@ -464,6 +473,12 @@ int mla_decode_launch(const MlaParams& p, cudaStream_t st) {
   if (p.bs < 1 || (p.bs & (p.bs - 1)) || p.splits < 1 || p.splits > 32) return -1;
   if (p.f32) return p.splits == 1 ? plain_e<float>(p, st) : -1;
   if (!mla_tensor_core_sizes(p.kv_lora, p.rope_pad)) return p.splits == 1 ? plain_e<__nv_bfloat16>(p, st) : -1;
+  if (mla_decode_tc_takes(p.kv_lora, p.rope_pad, p.bs, p.fine, p.scale)) {
+    const int rc = mla_decode_tc_launch(p, st);
+    if (rc != 0) return rc;
+    if (p.splits > 1) mla_combine_kernel<<<(p.T * p.H * 32 + 255) / 256, 256, 0, st>>>(p);
+    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  }
   switch (p.kv_lora) {
     case 64: return decode_fine<64>(p, st);
     case 128: return decode_fine<128>(p, st);

@@ -499,7 +499,7 @@ def choose_kv_splits(base_ctas: int, max_seq: int, num_sms: int) -> int:
     return max(1, min(want, by_ctx, 32))
 
 
-def choose_decode_splits(base_ctas: int, max_seq: int, num_sms: int, per_sm: int = 2) -> int:
+def choose_decode_splits(base_ctas: int, max_seq: int, num_sms: int, per_sm: int = 2, start: float = 1.6, tile: float = 1.9) -> int:
     """KV splits of the paged decode kernel from a cost model of its waves. ``per_sm`` CTAs fit per SM; a CTA needs about 1.6 us to start
     and 1.9 us per 64-key tile when the SMs are full, and more than one split adds the combine launch (about 6 us). Measured on
     B200 (64 requests x 8 KV heads x 1150 keys): 71.7 us unsplit against 80.9 us in two splits, whose 1024 CTAs need four waves
@@ -512,7 +512,7 @@ def choose_decode_splits(base_ctas: int, max_seq: int, num_sms: int, per_sm: int
         if s > 1 and per < 2:
             break
         waves = -(-(max(base_ctas, 1) * s) // slots)
-        cost = waves * (1.6 + 1.9 * per) + (6.0 + 0.15 * s if s > 1 else 0.0)  # the combine kernel reads one partial per split
+        cost = waves * (start + tile * per) + (6.0 + 0.15 * s if s > 1 else 0.0)  # the combine kernel reads one partial per split
         if best_cost is None or cost < best_cost - 1e-9:
             best, best_cost = s, cost
     return best
@@ -817,7 +817,11 @@ def per_head_matmul(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
 
 
 def plan_mla_splits(H: int, lora: int, query_lens: list, seq_lens: list, num_sms: int) -> int:
-    """KV splits of a latent-attention launch: as many CTAs fit an SM as two key tiles and the queries leave room for."""
+    """KV splits of a latent-attention launch: as many CTAs fit an SM as two key tiles and the queries leave room for. The tcgen05 kernel has
+    one CTA per SM and two of them (halves of the output columns) per 128 rows, which need about
+    6 us to start and 1.3 us per key tile (measured: 97 us at 32 requests x 4096 keys x 128 heads in two splits)."""
+    if _C.mla_decode_wide(lora):
+        return choose_decode_splits(2 * sum(-(-q * H // 128) for q in query_lens), max(seq_lens), num_sms, 1, start=6.0, tile=1.3)
     per_sm = max(1, min(4, (227 << 10) // ((16 + 2 * 64) * (lora + 64) * 2 + 6144)))
     return choose_decode_splits(len(query_lens) * -(-max(query_lens) * H // 16), max(seq_lens), num_sms, per_sm)
 
