@@ -694,6 +694,9 @@ static void moe_gemm_run(const torch::Tensor& in, const torch::Tensor& w, const 
   p.ws = nullptr; p.counters = (int*)counters.data_ptr(); p.max_counters = 0;
   p.work = wl; p.work_count = cnt; p.work_capacity = cap;
   p.tn = tn; p.num_t_tiles = 1; p.num_n_tiles = 1; p.splits = 1; p.ktiles_per_split = Kd / 64;
+  // light CTAs, two to an SM: at these tiles a CTA's time goes into the hand-over between its warps, not into products (fp8, 256 experts x 2048 x
+  // 512, 8 / 32 / 64 tokens each: 270 / 377 / 428 us for the layer where one CTA per SM took 350 / 505 / 564)
+  p.small = wkind != 0 && tn <= 64;
   oc::gemm_plan_stages(p, wkind != 0);
   int r = oc::gemm_launch(p, in.data_ptr(), (int)in.stride(0), wkind == 0 ? w.data_ptr() : nullptr, wkind == 0 ? (int)w.stride(0) : 0, sm_count(),
                           cur_stream());

@@ -796,8 +796,7 @@ void gemm_plan(GemmParams& p, int num_sms, bool w4) {
     if (forced == 128 || forced == 192) tn = forced;
   }
   p.tn = tn;
-  // decode-sized dense problems with packed weights run the light CTA variant, two per SM (grouped work lists keep the full one:
-  // their items are token slices of many experts and the list is sized for one CTA per SM)
+  // decode-sized dense problems with packed weights run the light CTA variant, two per SM (so do grouped ones, whose callers set it)
   p.small = (w4 && use_small && tn <= 64 && p.work == nullptr) ? 1 : 0;
   const int slots = p.small ? 2 * num_sms : num_sms;
   // packed weights and many token tiles: pair the token tiles so that every dequantised weight tile feeds two accumulators. With one
@@ -932,7 +931,7 @@ int gemm_launch(const GemmParams& p_in, const void* x, int ldx, const void* w_bf
   if (w4 && p.wkind == 0) p.wkind = 1;  // packed weights without a stated kind are 4-bit integer
   if (!w4) { p.wkind = 0; p.small = 0; }
   if (p.wkind < 0 || p.wkind > 4) return -6;
-  if (p.small && (p.tn > 64 || p.work != nullptr)) return -7;
+  if (p.small && p.tn > 64) return -7;
   int total = p.work != nullptr ? p.work_capacity : p.num_n_tiles * p.num_t_tiles * p.splits;
   const int slots = p.small ? 2 * num_sms : num_sms;
   int grid = total < slots ? total : slots;
