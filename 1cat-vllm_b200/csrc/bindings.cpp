@@ -87,6 +87,11 @@ void gemm(torch::Tensor x, c10::optional<torch::Tensor> w, c10::optional<torch::
   p.trace = (unsigned long long*)(uintptr_t)trace_ptr;
   p.push_sel = (const int*)(uintptr_t)push_sel;
   p.push_sel_stride = (long long)push_sel_stride;
+  if (force_splits <= 0 && force_tn <= 0 && oc::gemm_skinny_takes(p)) {
+    const int rc = oc::gemm_skinny_launch(p, x.data_ptr(), (int)x.stride(0), sm_count(), cur_stream());
+    TORCH_CHECK(rc == 0, "gemm launch failed with code ", rc);
+    return;
+  }
   oc::gemm_plan(p, sm_count(), w4.has_value());
   if (force_tn > 0) {
     TORCH_CHECK(!w4.has_value() || force_tn <= 192, "4-bit weights support token tiles up to 192");

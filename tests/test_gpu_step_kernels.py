@@ -74,3 +74,48 @@ def test_mla_decode_tiles_of_128_rows(qlens, ctxs, H, rope, options):
         out = K().mla_decode(q_abs.cuda(), q_pe.cuda(), cache.cuda(), md, 192 ** -0.5, lora, sinks=dev(sinks), gate=dev(gate))
         assert K().check_status() == 0
         _close(out, want, 2e-2, 5e-3)
+
+
+def _packed(kind, N, Kd, g):
+    """(packed tiles, scale table, padded rows, k tiles per group, weights in fp64) of random weights."""
+    n = 64 if Kd % 128 else 128   # group
+    if kind == 1:
+        q, z = torch.randint(0, 16, (N, Kd), generator=g, dtype=torch.uint8), torch.randint(0, 16, (N, Kd // n), generator=g, dtype=torch.uint8)
+        s = torch.rand(N, Kd // n, generator=g) * 0.01 + 0.001
+        w = ((q.float() - z.float().repeat_interleave(n, 1)) * s.bfloat16().float().repeat_interleave(n, 1)).bfloat16().double()
+        return (*K().pack_w4(q.cuda(), z.cuda(), s.cuda(), n), n // 64, w)
+    if kind == 2:
+        c = torch.randn(N, Kd, generator=g).to(torch.float8_e4m3fn)
+        s = torch.rand(N, Kd // n, generator=g) * 0.02 + 0.001
+        return (*K().pack_fp8(c.view(torch.uint8).cuda(), s.cuda(), n), n // 64, (c.float() * s.bfloat16().float().repeat_interleave(n, 1)).bfloat16().double())
+    c = torch.randint(0, 256, (N, Kd // 2), generator=g, dtype=torch.uint8)
+    values = torch.tensor([0, .5, 1, 1.5, 2, 3, 4, 6, 0, -.5, -1, -1.5, -2, -3, -4, -6], dtype=torch.float64)[torch.stack([c & 15, c >> 4], -1).long().flatten(1)]
+    if kind == 3:
+        e = torch.randint(119, 123, (N, Kd // 32), generator=g, dtype=torch.uint8)
+        return (*K().pack_mxfp4(c.cuda(), e.cuda()), 1, values * torch.exp2(e.double() - 127).repeat_interleave(32, 1))
+    s = (torch.rand(N, Kd // 16, generator=g) * 4 + 0.5).to(torch.float8_e4m3fn)
+    w = values * s.double().repeat_interleave(16, 1) * 0.25
+    return (*K().pack_nvfp4(c.cuda(), s.cuda(), torch.tensor(0.25).cuda()), 1, w)
+
+
+@pytest.mark.parametrize("kind", [1, 2, 3, 4])
+@pytest.mark.parametrize("T,N,Kd,gated", [(1, 128, 128, False), (8, 160, 1152, True), (9, 96, 4224, False), (16, 5120, 704, True), (3, 224, 64, True), (13, 64, 8320, False)])
+def test_gemm_of_a_few_tokens(kind, T, N, Kd, gated):
+    """One and two blocks of eight tokens, full and ragged, rows that end inside a tile, k ranges of an odd number of tiles, of fewer than the warps
+    and of many, gated and plain (with a bias) epilogues, a strided activation. Weights are rounded to bf16 where they are widened; fp32 sums, one rounding at the end."""
+    g = torch.Generator().manual_seed(kind * 100 + T)
+    tiles, sz, npad, gk, w = _packed(kind, N, Kd, g)
+    x = (torch.randn(T, Kd + 64, generator=g)).bfloat16()[:, :Kd]
+    y = x.double() @ w.t()
+    bias = None
+    if gated:
+        pair = y.view(T, -1, 2, 16)
+        want = (torch.nn.functional.silu(pair[:, :, 0]) * pair[:, :, 1]).reshape(T, -1)
+    else:
+        bias = torch.randn(N, generator=g).bfloat16()
+        want = y + bias.double()
+    out = torch.full((T + 1, want.shape[1] + 8), 7.0, dtype=torch.bfloat16, device="cuda")
+    K()._gemm(x.cuda(), None, tiles, sz, out[:T, : want.shape[1]], None if bias is None else bias.cuda(), N, N, want.shape[1], npad, 1 if gated else 0, gk, wkind=kind)
+    torch.cuda.synchronize()
+    assert (out[T:] == 7).all() and (out[:, want.shape[1]:] == 7).all()
+    _close(out[:T, : want.shape[1]], want, 2 ** -6, float(want.abs().mean()) * 2 ** -6, f"kind {kind}")
