@@ -11,7 +11,7 @@
 // Options for the Gemma / GPT-OSS / Mistral families: a sliding window (a query at position i sees keys i-window+1 .. i; key tiles
 // wholly before the window are skipped), tanh soft-capping of the scaled scores, and per-head attention sinks (a learned logit that
 // joins the softmax denominator only).
-// FP8 KV cache (KV8): pages hold e4m3 bytes in the same layout; tiles stream through a byte-wide cp.async ring and are widened to
+// FP8 KV cache (KV8; decoding with heads of 128 and 256 runs attention_fp8.cu instead): pages hold e4m3 bytes in the same layout; tiles stream through a byte-wide cp.async ring and are widened to
 // bf16 into one working tile per operand before the MMAs; the per-tensor scales fold into the softmax scale (K) and the output (V).
 // Extended variants (EXT, bf16 cache): first tokens that stay visible outside the window (their tiles are walked ahead of the window's),
 // a bias by distance added to the scores in fp32, values that are the keys (one tensor per page: the ring holds one tile per stage and
@@ -759,19 +759,34 @@ __global__ void attn_combine_kernel(const AttnParams p) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int rows = p.T * p.Hq;
   if (warp >= rows) return;
+  // a lane per split for maxima and sums, then four splits' rows in flight
   float M = -INFINITY;
-  for (int s = 0; s < p.splits; ++s) M = fmaxf(M, p.ws_ml[((size_t)s * rows + warp) * 2]);
+  for (int s = lane; s < p.splits; s += 32) M = fmaxf(M, p.ws_ml[((size_t)s * rows + warp) * 2]);
+  M = warp_max(M);
   float L = 0.f;
   float acc[D / 32];
 #pragma unroll
   for (int i = 0; i < D / 32; ++i) acc[i] = 0.f;
-  for (int s = 0; s < p.splits; ++s) {
-    const float ms = p.ws_ml[((size_t)s * rows + warp) * 2];
-    const float f = (ms == -INFINITY) ? 0.f : exp2f(ms - M);
-    L += p.ws_ml[((size_t)s * rows + warp) * 2 + 1] * f;
-    const float* src = p.ws_o + ((size_t)s * rows + warp) * D;
+  for (int s0 = 0; s0 < p.splits; s0 += 32) {
+    const int ns = min(32, p.splits - s0);
+    const float* ml = p.ws_ml + ((size_t)(s0 + lane) * rows + warp) * 2;
+    const float mine = lane < ns && ml[0] != -INFINITY ? exp2f(ml[0] - M) : 0.f;
+    L += warp_sum(lane < ns ? ml[1] * mine : 0.f);
+    for (int s = 0; s < ns; s += 4) {
+      float v[4][D / 32], f[4];
 #pragma unroll
-    for (int i = 0; i < D / 32; ++i) acc[i] += src[lane + 32 * i] * f;
+      for (int u = 0; u < 4; ++u) {
+        f[u] = __shfl_sync(0xffffffffu, mine, (s + u) & 31);
+        const float* src = p.ws_o + ((size_t)(s0 + min(s + u, ns - 1)) * rows + warp) * D;
+        if (s + u >= ns) f[u] = 0.f;
+#pragma unroll
+        for (int i = 0; i < D / 32; ++i) v[u][i] = src[lane + 32 * i];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int i = 0; i < D / 32; ++i) acc[i] += v[u][i] * f[u];
+    }
   }
   const float den = L + (p.sinks != nullptr ? exp2f(p.sinks[warp % p.Hq] * 1.4426950408889634f - M) : 0.f);
   const float inv = (den > 0.f ? (p.kv_fp8 ? p.v_scale : 1.f) / den : 0.f) * head_gate(p, (size_t)(warp / p.Hq), warp % p.Hq);
@@ -816,6 +831,12 @@ __global__ void diff_combine_kernel(const AttnParams p) {
     if (lane + 32 * i < p.vdim) p.out[(size_t)warp * p.vdim + lane + 32 * i] = __float2bfloat16(x[i] * g);
 }
 
+template <int D>
+int combine(const AttnParams& p, cudaStream_t st) {
+  if (p.splits > 1) launch_k(attn_combine_kernel<D>, dim3((p.T * p.Hq * 32 + 255) / 256), dim3(256), 0, st, true, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
 template <int D, int MODE, int MB, bool KV8, int ST = 3, bool EXT = false, bool DIFF = false>
 int launch_one(const AttnParams& p, cudaStream_t st) {
   constexpr int ROWS = (MODE == 0) ? 64 : 16 * MB;
@@ -835,9 +856,8 @@ int launch_one(const AttnParams& p, cudaStream_t st) {
   if (grid.x == 0) return 0;
   launch_k(attn_kernel<D, MODE, MB, KV8, ST, EXT, DIFF>, grid, dim3(128), (size_t)smem, st, true, p);
   if (MODE == 1 && p.splits > 1) {
-    int rows = p.T * p.Hq;
-    if constexpr (DIFF) launch_k(diff_combine_kernel<D>, dim3((rows / 2 * 32 + 255) / 256), dim3(256), 0, st, true, p);
-    else launch_k(attn_combine_kernel<D>, dim3((rows * 32 + 255) / 256), dim3(256), 0, st, true, p);
+    if constexpr (DIFF) launch_k(diff_combine_kernel<D>, dim3((p.T * p.Hq / 2 * 32 + 255) / 256), dim3(256), 0, st, true, p);
+    else return combine<D>(p, st);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -888,19 +908,22 @@ int attention_launch(const AttnParams& p, int mode, cudaStream_t st) {
   }
   if (mode == 1) {
     const int rows = p.short_q_len * G;
+    if (f8 && p.D != 64) {
+      const int rc = attention_decode_fp8_launch(p, st);
+      return rc != 0 ? rc : (p.D == 128 ? combine<128>(p, st) : combine<256>(p, st));
+    }
     if (p.D == 64) {
       if (rows <= 16) return f8 ? launch_one<64, 1, 1, true>(p, st) : launch_one<64, 1, 1, false>(p, st);
       if (rows <= 32) return f8 ? launch_one<64, 1, 2, true>(p, st) : launch_one<64, 1, 2, false>(p, st);
     } else if (p.D == 128) {
       if (rows <= 16) {
-        if (f8) return launch_one<128, 1, 1, true>(p, st);
         // two ring stages leave room for a third CTA per SM (experiment switch; three stages and two CTAs are the default)
         static const int two_stage = getenv("ONECAT_ATTN_STAGES") && atoi(getenv("ONECAT_ATTN_STAGES")) == 2;
         return two_stage ? launch_one<128, 1, 1, false, 2>(p, st) : launch_one<128, 1, 1, false>(p, st);
       }
-      if (rows <= 32) return f8 ? launch_one<128, 1, 2, true>(p, st) : launch_one<128, 1, 2, false>(p, st);
+      if (rows <= 32) return launch_one<128, 1, 2, false>(p, st);
     } else {
-      if (rows <= 16) return f8 ? launch_one<256, 1, 1, true>(p, st) : launch_one<256, 1, 1, false>(p, st);
+      if (rows <= 16) return launch_one<256, 1, 1, false>(p, st);
     }
     return -6;  // caller must use mode 0 for longer queries
   }

@@ -129,6 +129,7 @@ int attention_f32_launch(const AttnParams& p, bool bf16, cudaStream_t st);
 // mode 0: rows of a query tile are spread over warps (prefill / long queries); mode 1: keys are spread over warps
 // (decode and short verify queries, with split-KV + combine).
 int attention_launch(const AttnParams& p, int mode, cudaStream_t st);
+int attention_decode_fp8_launch(const AttnParams& p, cudaStream_t st);   // its decode mode over an fp8 cache, heads of 128 and 256
 unsigned int attention_read_status(bool clear);
 void attention_read_status_async(unsigned int* dst, cudaStream_t st);
 // Differential attention ahead of its kernels: per (token, head, map) RMS norm and rotation of queries and keys, cache insert.

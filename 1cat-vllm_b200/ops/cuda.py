@@ -519,7 +519,7 @@ def choose_decode_splits(base_ctas: int, max_seq: int, num_sms: int, per_sm: int
 
 
 def plan_attention(query_lens: list, seq_lens: list, Hq: int, Hkv: int, D: int, num_sms: int, force_splits: int = 0, span: int = 0,
-                   extended: bool = False):
+                   extended: bool = False, fp8: bool = False):
     """Decide which requests take the decode kernel (rows = q_len * group fit in one 16/32-row tile) and how many KV
     splits it uses. Returns (short_q_len, num_q_tiles for the prefill kernel, splits). ``span`` > 0: a decode row reads at most that many
     keys of its context (window and kept first tokens). ``extended``: the variants of the kernel with one ring of shared keys and values,
@@ -536,7 +536,9 @@ def plan_attention(query_lens: list, seq_lens: list, Hq: int, Hkv: int, D: int, 
     if n_short:
         max_s = max((s for q, s in zip(query_lens, seq_lens) if q <= short), default=1)
         per_sm = {64: 5, 128: 4}.get(D, 2) if extended and short * G <= 16 else 2
-        splits = choose_decode_splits(n_short * Hkv, min(max_s, span) if span else max_s, num_sms, per_sm)
+        # attention_fp8.cu: three CTAs per SM for heads of 128, two for 256; its times measured with full SMs
+        cost = dict(per_sm=3 if D == 128 and short * G <= 16 else 2, start=5.0, tile=1.35) if fp8 and D >= 128 else dict(per_sm=per_sm)
+        splits = choose_decode_splits(n_short * Hkv, min(max_s, span) if span else max_s, num_sms, **cost)
     if force_splits:
         splits = force_splits
     return short, tiles, splits
@@ -568,7 +570,7 @@ def paged_attention(q, kv_cache, md, scale, out=None, lse=None, window=0, softca
     plan = getattr(md, "attn_plan", None)
     if plan is None or plan[0] != key:
         plan = (key, plan_attention(md.query_lens_cpu, md.seq_lens_cpu, Hq, Hkv, D, _sms(q.device), span=key[3] if extended else 0,
-                                    extended=kv_cache.shape[1] == 1))
+                                    extended=kv_cache.shape[1] == 1, fp8=kv_cache.dtype == torch.float8_e4m3fn))
         md.attn_plan = plan
     short, tiles, splits = plan[1]
     n_short = sum(1 for x in md.query_lens_cpu if 0 < x <= short)

@@ -119,3 +119,36 @@ def test_gemm_of_a_few_tokens(kind, T, N, Kd, gated):
     torch.cuda.synchronize()
     assert (out[T:] == 7).all() and (out[:, want.shape[1]:] == 7).all()
     _close(out[:T, : want.shape[1]], want, 2 ** -6, float(want.abs().mean()) * 2 ** -6, f"kind {kind}")
+
+
+@pytest.mark.parametrize("D,Hq,Hkv,qlens,ctxs,options", [
+    (128, 40, 8, [1, 1, 1], [0, 31, 5000], {}), (128, 8, 8, [1] * 5, [127, 128, 129, 15, 700], dict(softcap=20.0)), (128, 16, 1, [1, 1], [3000, 64], dict(sinks=True)),
+    (128, 32, 4, [4, 1, 2], [95, 4000, 17], {}), (128, 6, 2, [3, 3], [600, 40], dict(window=100)), (256, 24, 4, [1, 2, 1], [0, 1000, 63], dict(window=70, softcap=30.0)),
+    (256, 16, 2, [1, 1], [8000, 33], dict(sinks=True)), (256, 16, 4, [4, 3], [2000, 1], {})])
+def test_decode_over_an_fp8_cache(D, Hq, Hkv, qlens, ctxs, options):
+    """One and two blocks of 16 rows, turns that end with the context, in one and several splits, windows, caps and sinks; the bytes past a context
+    are those of the largest codes. Queries and weights are bf16 (2^-8 each)."""
+    from onecat_vllm.worker.attn_metadata import AttentionMetadata
+    bs, R, T = 16, len(qlens), sum(qlens)
+    g = torch.Generator().manual_seed(D + Hq)
+    seq = [c + q for q, c in zip(qlens, ctxs)]
+    per = [-(-s // bs) for s in seq]
+    bt, at = torch.zeros(R, max(per) + 1, dtype=torch.int32), 1
+    cache = torch.randn(sum(per) + 1, 2, Hkv, bs, D, generator=g).to(torch.float8_e4m3fn)
+    for r, n in enumerate(per):
+        bt[r, :n] = torch.arange(at, at + n, dtype=torch.int32).flip(0)
+        at += n
+        if seq[r] % bs:
+            cache.view(torch.uint8)[bt[r, n - 1].long(), :, :, seq[r] % bs:] = 0x7e
+    q = torch.randn(T, Hq, D, generator=g).bfloat16()
+    window, softcap = options.get("window", 0), options.get("softcap", 0.0)
+    sinks = torch.randn(Hq, generator=g) if options.get("sinks") else None
+    qsl, sl = torch.tensor([0, *torch.tensor(qlens).cumsum(0).tolist()], dtype=torch.int32), torch.tensor(seq, dtype=torch.int32)
+    want = ref.paged_attention(q, cache, bt, qsl, sl, D ** -0.5, window=window, softcap=softcap, sinks=sinks)
+    for splits in (1, 3, None):
+        md = AttentionMetadata(R, T, qsl.cuda(), sl.cuda(), bt.cuda(), None, None, max(qlens), max(seq), query_lens_cpu=list(qlens), seq_lens_cpu=seq)
+        if splits:
+            md.attn_plan = ((Hq, Hkv, D), (max(qlens), 0, splits))
+        out = K().paged_attention(q.cuda(), cache.cuda(), md, D ** -0.5, window=window, softcap=softcap, sinks=None if sinks is None else sinks.cuda())
+        assert K().check_status() == 0
+        _close(out, want, 2e-2, 1e-2, f"{splits} splits")
