@@ -585,8 +585,8 @@ def paged_attention(q, kv_cache, md, scale, out=None, lse=None, window=0, softca
     if tiles:
         if (D == 128 and q.stride(1) == D and _ATTN_PREFILL_TC and not window and not softcap and sinks is None and not extended
                 and kv_cache.dtype == torch.bfloat16):
-            # tcgen05 kernel: 128-token query tiles per (request, head)
-            tiles_tc = sum(-(-x // 128) for x in md.query_lens_cpu if x > short)
+            # tcgen05 kernel: 256 query tokens per CTA
+            tiles_tc = sum(-(-x // 256) for x in md.query_lens_cpu if x > short)
             _C.paged_attention(q, kv_cache, out, lse, md.query_start_loc, md.seq_lens, md.block_table, scale, 2, tiles_tc, 1,
                                md.max_query_len, short, None, None, 0, 0.0, None, 1.0, 1.0)
         else:

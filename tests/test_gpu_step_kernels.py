@@ -152,3 +152,31 @@ def test_decode_over_an_fp8_cache(D, Hq, Hkv, qlens, ctxs, options):
         out = K().paged_attention(q.cuda(), cache.cuda(), md, D ** -0.5, window=window, softcap=softcap, sinks=None if sinks is None else sinks.cuda())
         assert K().check_status() == 0
         _close(out, want, 2e-2, 1e-2, f"{splits} splits")
+
+
+@pytest.mark.parametrize("qlens,ctxs,Hq,Hkv,scale", [([256, 257, 1, 128], [0, 1, 500, 128], 8, 2, 1.0), ([129, 640, 17], [127, 300, 2000], 4, 4, 1.0), ([700], [0], 2, 1, 30.0)])
+def test_prompt_attention_in_pairs_of_query_tiles(qlens, ctxs, Hq, Hkv, scale):
+    """Portions that end inside the first or the second tile of a pair, one that fills both, tiles of unequal numbers of key tiles, a decoding request
+    beside them, and scores that grow by far more than 2^8 along a row (the accumulator is rescaled). Weights are bf16 (2^-8)."""
+    from onecat_vllm.worker.attn_metadata import AttentionMetadata
+    D, bs, R, T = 128, 16, len(qlens), sum(qlens)
+    g = torch.Generator().manual_seed(T)
+    seq = [c + q for q, c in zip(qlens, ctxs)]
+    per = [-(-s // bs) for s in seq]
+    bt, at = torch.zeros(R, max(per), dtype=torch.int32), 1
+    for r, n in enumerate(per):
+        bt[r, :n] = torch.arange(at, at + n, dtype=torch.int32).flip(0)
+        at += n
+    cache = torch.randn(at, 2, Hkv, bs, D, generator=g)
+    if scale != 1.0:   # keys grow with their position
+        order = bt[0].long()
+        cache[order, 0] *= torch.linspace(0.1, scale, len(order)).view(-1, 1, 1, 1)
+    cache, q = cache.bfloat16(), torch.randn(T, Hq, D, generator=g).bfloat16()
+    qsl, sl = torch.tensor([0, *torch.tensor(qlens).cumsum(0).tolist()], dtype=torch.int32), torch.tensor(seq, dtype=torch.int32)
+    md = AttentionMetadata(R, T, qsl.cuda(), sl.cuda(), bt.cuda(), None, None, max(qlens), max(seq), query_lens_cpu=list(qlens), seq_lens_cpu=seq)
+    lse = torch.zeros(T, Hq, device="cuda")
+    out = K().paged_attention(q.cuda(), cache.cuda(), md, D ** -0.5, lse=lse)
+    assert K().check_status() == 0
+    _close(out, ref.paged_attention(q, cache, bt, qsl, sl, D ** -0.5), 2e-2, 1e-2)
+    s = torch.einsum("hd,kd->hk", q[qsl[1] - 1, : Hq // Hkv].float(), cache[bt[0, :per[0]].long(), 0, 0].reshape(-1, D)[: seq[0]].float()) * D ** -0.5
+    _close(lse[qsl[1] - 1, : Hq // Hkv], torch.logsumexp(s, -1), 1e-3, 1e-2, "lse")
