@@ -92,6 +92,11 @@ void gemm(torch::Tensor x, c10::optional<torch::Tensor> w, c10::optional<torch::
     TORCH_CHECK(rc == 0, "gemm launch failed with code ", rc);
     return;
   }
+  if (force_splits <= 0 && force_tn <= 0 && !w4.has_value() && oc::gemm_pair_takes(p, sm_count())) {
+    const int rc = oc::gemm_pair_launch(p, x.data_ptr(), (int)x.stride(0), wptr, ldw, sm_count(), cur_stream());
+    TORCH_CHECK(rc == 0, "gemm launch failed with code ", rc);
+    return;
+  }
   oc::gemm_plan(p, sm_count(), w4.has_value());
   if (force_tn > 0) {
     TORCH_CHECK(!w4.has_value() || force_tn <= 192, "4-bit weights support token tiles up to 192");
@@ -1281,10 +1286,11 @@ void read_status_async(torch::Tensor pinned) {
   oc::diff_prefill_read_status_async(p + 11, st);
   oc::talk_prefill_read_status_async(p + 12, st);
   oc::mla_decode_tc_read_status_async(p + 13, st);
+  oc::gemm_pair_read_status_async(p + 14, st);
 }
 
 int64_t read_status(bool clear) {
-  return (int64_t)(oc::gemm_read_status(clear) | oc::elementwise_read_status(clear) | oc::attention_read_status(clear) | oc::attention_tc_read_status(clear) |
+  return (int64_t)(oc::gemm_read_status(clear) | oc::gemm_pair_read_status(clear) | oc::elementwise_read_status(clear) | oc::attention_read_status(clear) | oc::attention_tc_read_status(clear) |
                    oc::comm_read_status(clear) | oc::gdn_read_status(clear) | oc::sampling_read_status(clear) | oc::moe_read_status(clear) | oc::mla_read_status(clear) | oc::mla_decode_tc_read_status(clear) | oc::mla_prefill_read_status(clear) | oc::diff_prefill_read_status(clear) | oc::talk_prefill_read_status(clear) | oc::ep_read_status(clear));
 }
 

@@ -57,6 +57,11 @@ void gemm_plan(GemmParams& p, int num_sms, bool w4);
 void gemm_plan_stages(GemmParams& p, bool w4);
 int gemm_smem_bytes(const GemmParams& p);
 int gemm_launch(const GemmParams& p, const void* x, int ldx, const void* w_bf16, int ldw, int num_sms, cudaStream_t stream);
+// many tokens, bf16 weights, pairs of SMs (gemm_pair.cu)
+bool gemm_pair_takes(const GemmParams& p, int num_sms);
+int gemm_pair_launch(const GemmParams& p, const void* x, int ldx, const void* w, int ldw, int num_sms, cudaStream_t stream);
+unsigned int gemm_pair_read_status(bool clear);
+void gemm_pair_read_status_async(unsigned int* dst, cudaStream_t st);
 // a few tokens, packed weights (gemm_skinny.cu)
 bool gemm_skinny_takes(const GemmParams& p);
 int gemm_skinny_launch(const GemmParams& p, const void* x, int ldx, int num_sms, cudaStream_t stream);

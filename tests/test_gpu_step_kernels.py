@@ -180,3 +180,30 @@ def test_prompt_attention_in_pairs_of_query_tiles(qlens, ctxs, Hq, Hkv, scale):
     _close(out, ref.paged_attention(q, cache, bt, qsl, sl, D ** -0.5), 2e-2, 1e-2)
     s = torch.einsum("hd,kd->hk", q[qsl[1] - 1, : Hq // Hkv].float(), cache[bt[0, :per[0]].long(), 0, 0].reshape(-1, D)[: seq[0]].float()) * D ** -0.5
     _close(lse[qsl[1] - 1, : Hq // Hkv], torch.logsumexp(s, -1), 1e-3, 1e-2, "lse")
+
+
+@pytest.mark.parametrize("T,N,Kd,epi,bias,f32", [(256, 9472, 64, 0, False, False), (300, 5120, 640, 0, True, False), (2500, 1000, 1088, 0, True, True), (129, 9600, 128, 1, False, False),
+                                                 (1030, 2112, 448, 3, False, False), (515, 3336, 192, 2, True, False), (9000, 520, 256, 0, False, False)])
+def test_gemm_over_pairs_of_sms(T, N, Kd, epi, bias, f32):
+    """Ragged tokens and features, rings shorter and longer than the k tiles, several tiles per pair of SMs, a last group of fewer token tiles; plain, gated
+    and activated epilogues, fp32 and bf16 results. One rounding of an fp32 sum."""
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, Kd + 64, device="cuda", generator=g).bfloat16()[:, :Kd]
+    w = (torch.randn(N, Kd, device="cuda", generator=g) * Kd ** -0.5).bfloat16()
+    b = torch.randn(N, device="cuda", generator=g).bfloat16() if bias else None
+    y = x.double() @ w.double().t()
+    if epi in (1, 3):
+        pair = y.view(T, -1, 2, 16)
+        act = torch.nn.functional.silu(pair[:, :, 0]) if epi == 1 else torch.nn.functional.gelu(pair[:, :, 0], approximate="tanh")
+        want = (act * pair[:, :, 1]).reshape(T, -1)
+    else:
+        want = y if b is None else y + b.double()
+        want = torch.nn.functional.gelu(want, approximate="tanh") if epi == 2 else want
+    n = want.shape[1]
+    out = torch.full((T + 1, n + 8), 7.0, dtype=torch.float32 if f32 else torch.bfloat16, device="cuda")
+    before = K().check_status()
+    K()._gemm(x, w, None, None, out[:T, :n], b, N, N, n, 0, epi, 1)
+    torch.cuda.synchronize()
+    assert before == 0 and K().check_status() == 0
+    assert (out[T:] == 7).all() and (out[:, n:] == 7).all()
+    _close(out[:T, :n], want, 1e-4 if f32 else 2 ** -7, 1e-4 if f32 else 2 ** -9)
