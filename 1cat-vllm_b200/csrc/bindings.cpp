@@ -92,6 +92,12 @@ void gemm(torch::Tensor x, c10::optional<torch::Tensor> w, c10::optional<torch::
     TORCH_CHECK(rc == 0, "gemm launch failed with code ", rc);
     return;
   }
+  if (force_splits <= 0 && force_tn <= 0 && oc::gemm_widen_takes(p, sm_count())) {
+    auto slab = torch::empty({oc::gemm_widen_rows(p, sm_count()), p.K}, x.options());
+    const int rc = oc::gemm_widen_launch(p, x.data_ptr(), (int)x.stride(0), slab.data_ptr(), sm_count(), cur_stream());
+    TORCH_CHECK(rc == 0, "gemm launch failed with code ", rc);
+    return;
+  }
   if (force_splits <= 0 && force_tn <= 0 && !w4.has_value() && oc::gemm_pair_takes(p, sm_count())) {
     const int rc = oc::gemm_pair_launch(p, x.data_ptr(), (int)x.stride(0), wptr, ldw, sm_count(), cur_stream());
     TORCH_CHECK(rc == 0, "gemm launch failed with code ", rc);

@@ -25,6 +25,7 @@ constexpr int kHalfBytes = 128 * 128;             // 128 rows x 64 k of bf16
 constexpr int kStage = 2 * kHalfBytes, kStages = 6;
 constexpr int kThreads = 192;
 constexpr int kSmem = kStages * kStage + 1024 + 1024;
+constexpr int kWidenTokens = 1024;                // see gemm_widen_takes
 constexpr int kGroup = 8;                         // token tiles of a group
 
 __device__ __forceinline__ float gelu_tanh(float z) {
@@ -301,6 +302,117 @@ int gemm_pair_launch(const GemmParams& p_in, const void* x, int ldx, const void*
   const int clusters = (int)(total < num_sms / 2 ? total : num_sms / 2);
   if (launch_k(gemm_pair_kernel, dim3(2 * clusters), dim3(kThreads), (size_t)kSmem, st, true, tmX, tmW, p) != cudaSuccess) return -10;
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
+// ---- packed weights, many tokens: rows [row0, row0 + rows) widened to bf16 [rows][K], a thread per eight neighbouring k. The numbers are those of
+// the widening inside gemm_sm100.cu.
+namespace {
+
+template <int WKIND>
+__global__ void __launch_bounds__(256) widen_kernel(const uint8_t* __restrict__ w, const uint32_t* __restrict__ sz, __nv_bfloat16* __restrict__ out, int row0,
+                                                    int K, int n_pad, int gk) {
+  constexpr int kTileBytes = WKIND == 2 ? 8192 : 4096, kScaleWords = WKIND == 4 ? 2 : 1, U = 4;
+  pdl_trigger();
+  pdl_wait();                             // the slab may still be read by the product before
+  const int c = threadIdx.x & 7, local = blockIdx.x * 32 + (threadIdx.x >> 3), row = row0 + local, ktiles = K / 64;
+  const int kt0 = blockIdx.y * U, rt = row & 127;
+  const uint8_t* src = w + (size_t)(row >> 7) * ktiles * kTileBytes + (WKIND == 2 ? (c >> 1) * 2048 + rt * 16 + (c & 1) * 8 : (c >> 2) * 2048 + rt * 16 + (c & 3) * 4);
+  uint32_t q[U][2], s[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int kt = min(kt0 + u, ktiles - 1);
+    if constexpr (WKIND == 2) {
+      const uint2 v = __ldcs(reinterpret_cast<const uint2*>(src + (size_t)kt * kTileBytes));
+      q[u][0] = v.x;
+      q[u][1] = v.y;
+    } else {
+      q[u][0] = __ldcs(reinterpret_cast<const uint32_t*>(src + (size_t)kt * kTileBytes));
+    }
+    s[u] = __ldg(sz + ((size_t)(kt / gk) * n_pad + row) * kScaleWords + (WKIND == 4 ? c >> 2 : 0));
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (kt0 + u >= ktiles) break;
+    // the scale of these k: int4 and fp8 one per tile, MXFP4 one per half, NVFP4 one per two words
+    const bool upper = WKIND == 3 ? c >= 4 : (WKIND == 4 ? (c & 2) : false);
+    const uint32_t sc = upper ? __byte_perm(s[u], 0, 0x3232) : __byte_perm(s[u], 0, 0x1010), z = __byte_perm(s[u], 0, 0x3232);
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      uint32_t v;
+      if constexpr (WKIND == 1) {
+        const uint32_t x = ((q[u][0] >> (4 * i)) & 0x000f000fu) | 0x43004300u;
+        const __nv_bfloat162 d = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&x), *reinterpret_cast<const __nv_bfloat162*>(&z));
+        v = *reinterpret_cast<const uint32_t*>(&d);
+      } else if constexpr (WKIND == 2) {
+        const uint32_t t = __byte_perm(q[u][i >> 1], 0, (i & 1) ? 0x3424 : 0x1404);
+        v = (t & 0x80008000u) | ((t >> 4) & 0x07f007f0u);
+      } else {
+        const uint32_t x = q[u][0] >> (4 * i);
+        v = ((x & 0x00080008u) << 12) | ((x & 0x00070007u) << 6);
+      }
+      const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&v), *reinterpret_cast<const __nv_bfloat162*>(&sc));
+      o[i] = *reinterpret_cast<const uint32_t*>(&r);
+    }
+    *reinterpret_cast<uint4*>(out + (size_t)local * K + (kt0 + u) * 64 + c * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
+}  // namespace
+
+// Feature tiles of a slab and the whole product's estimated time in us. A pair of SMs takes 0.38 us per k tile, every slab about 15 us of its own
+// (two launches, first copies, last tiles, the widening's tail), the widening moves 2.5 bytes a weight at 4 TB/s. Slabs are at most 192 MB.
+namespace {
+struct Slabs { int tiles; double us; };
+Slabs plan_slabs(const GemmParams& p, int num_sms) {
+  const int tt = (p.T + kTok - 1) / kTok, nt = (p.n_rows + kFeat - 1) / kFeat, pairs = num_sms / 2;
+  const long long tile_bytes = (long long)kFeat * p.K * 2;
+  Slabs best{1, 1e30};
+  for (int n = 1; n <= nt && (n == 1 || n * tile_bytes <= (192ll << 20)); ++n) {
+    const int slabs = (nt + n - 1) / n, rest = nt - (slabs - 1) * n;
+    const long long waves = (long long)(slabs - 1) * ((n * tt + pairs - 1) / pairs) + (rest * tt + pairs - 1) / pairs;
+    const double us = waves * (p.K / 64) * 0.38 + slabs * 15.0 + (double)p.n_rows * p.K * 2.5 / 4e6;
+    if (us < best.us) best = {n, us};
+  }
+  return best;
+}
+}  // namespace
+
+int gemm_widen_rows(const GemmParams& p, int num_sms) { return plan_slabs(p, num_sms).tiles * kFeat; }
+
+// Packed weights and many tokens: widening them once and running the pairs of SMs at 1.6 PFLOP/s, or widening tile by tile on the way into tensor
+// memory (gemm_sm100.cu, about 1.1 PFLOP/s: 0.72 us per k tile of 128 x 384, 0.45 of 128 x 192, and 20 us around them). The first only where
+// these estimates say that it wins by 5 %. Measured (us), int4: 34816 x 5120 at 8192 tokens 1939 for 2730, at 1087 tokens 520 for 383 in small
+// slabs; 5120 x 17408 at 1087 tokens 400 for 187.
+bool gemm_widen_takes(const GemmParams& p, int num_sms) {
+  if (p.w4 == nullptr || p.wkind < 1 || p.wkind > 4 || p.T < kWidenTokens || !gemm_pair_takes(p, num_sms)) return false;
+  const long long n = (p.n_rows + 127) / 128, w1 = (n * ((p.T + 191) / 192) + num_sms - 1) / num_sms, w2 = (n * ((p.T + 383) / 384) + num_sms - 1) / num_sms;
+  const double one = w1 * 0.45, two = w2 * 0.72, tile_by_tile = (p.K / 64) * (one < two ? one : two) + 20.0;
+  return plan_slabs(p, num_sms).us < 0.95 * tile_by_tile;
+}
+
+// The product over slabs of widened rows; `slab` holds gemm_widen_rows x K bf16.
+int gemm_widen_launch(const GemmParams& p, const void* x, int ldx, void* slab, int num_sms, cudaStream_t st) {
+  const int step = gemm_widen_rows(p, num_sms);
+  const bool gated = p.epi == EPI_SILU_MUL || p.epi == EPI_GELU_MUL;
+  for (int row0 = 0; row0 < p.n_rows; row0 += step) {
+    const int rows = p.n_rows - row0 < step ? p.n_rows - row0 : step;
+    const dim3 grid((rows + 31) / 32, (p.K / 64 + 3) / 4);   // rows past the last tile do not exist: a slab's rows end with it
+    auto widen = [&](auto kernel) {
+      return launch_k(kernel, grid, dim3(256), 0, st, true, p.w4, p.w4_sz, reinterpret_cast<__nv_bfloat16*>(slab), row0, p.K, p.n_pad, p.group_ktiles) == cudaSuccess;
+    };
+    const bool ok = p.wkind == 1 ? widen(widen_kernel<1>) : p.wkind == 2 ? widen(widen_kernel<2>) : p.wkind == 3 ? widen(widen_kernel<3>) : widen(widen_kernel<4>);
+    if (!ok) return -10;
+    GemmParams q = p;
+    q.n_rows = rows;
+    q.out = p.out + (gated ? row0 / 2 : row0);
+    q.N = p.N - row0 < rows ? p.N - row0 : rows;
+    q.n_out = p.n_out - row0 / 2;
+    if (p.bias != nullptr) q.bias = p.bias + row0;
+    const int rc = gemm_pair_launch(q, x, ldx, slab, p.K, num_sms, st);
+    if (rc != 0) return rc;
+  }
+  return 0;
 }
 
 unsigned int gemm_pair_read_status(bool clear) { return read_status_tu(clear); }

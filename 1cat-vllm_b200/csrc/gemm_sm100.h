@@ -60,6 +60,10 @@ int gemm_launch(const GemmParams& p, const void* x, int ldx, const void* w_bf16,
 // many tokens, bf16 weights, pairs of SMs (gemm_pair.cu)
 bool gemm_pair_takes(const GemmParams& p, int num_sms);
 int gemm_pair_launch(const GemmParams& p, const void* x, int ldx, const void* w, int ldw, int num_sms, cudaStream_t stream);
+// the same for packed weights, widened slab by slab
+bool gemm_widen_takes(const GemmParams& p, int num_sms);
+int gemm_widen_rows(const GemmParams& p, int num_sms);
+int gemm_widen_launch(const GemmParams& p, const void* x, int ldx, void* slab, int num_sms, cudaStream_t st);
 unsigned int gemm_pair_read_status(bool clear);
 void gemm_pair_read_status_async(unsigned int* dst, cudaStream_t st);
 // a few tokens, packed weights (gemm_skinny.cu)

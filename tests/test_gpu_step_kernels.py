@@ -207,3 +207,26 @@ def test_gemm_over_pairs_of_sms(T, N, Kd, epi, bias, f32):
     assert before == 0 and K().check_status() == 0
     assert (out[T:] == 7).all() and (out[:, n:] == 7).all()
     _close(out[:T, :n], want, 1e-4 if f32 else 2 ** -7, 1e-4 if f32 else 2 ** -9)
+
+
+@pytest.mark.parametrize("kind", [1, 2, 3, 4])
+@pytest.mark.parametrize("T,N,Kd,gated", [(1100, 5120, 192, True), (2048, 1312, 704, False), (1024, 9984, 4224, False)])
+def test_packed_gemm_of_many_tokens(kind, T, N, Kd, gated):
+    """One slab of widened weights and several (5888 rows of 4224 k each), rows that end inside a tile, odd numbers of k tiles. Weights are rounded to bf16 where
+    they are widened; fp32 sums, one rounding at the end."""
+    g = torch.Generator().manual_seed(kind + T)
+    tiles, sz, npad, gk, w = _packed(kind, N, Kd, g)
+    x = torch.randn(T, Kd, generator=g).bfloat16().cuda()
+    y = x.double() @ w.cuda().t()
+    bias = None
+    if gated:
+        pair = y.view(T, -1, 2, 16)
+        want = (torch.nn.functional.silu(pair[:, :, 0]) * pair[:, :, 1]).reshape(T, -1)
+    else:
+        bias = torch.randn(N, generator=g).bfloat16().cuda()
+        want = y + bias.double()
+    out = torch.full((T + 1, want.shape[1] + 8), 7.0, dtype=torch.bfloat16, device="cuda")
+    K()._gemm(x, None, tiles, sz, out[:T, : want.shape[1]], bias, N, N, want.shape[1], npad, 1 if gated else 0, gk, wkind=kind)
+    torch.cuda.synchronize()
+    assert K().check_status() == 0 and (out[T:] == 7).all() and (out[:, want.shape[1]:] == 7).all()
+    _close(out[:T, : want.shape[1]], want, 2 ** -6, float(want.abs().mean()) * 2 ** -6, f"kind {kind}")
