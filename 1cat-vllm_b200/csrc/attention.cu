@@ -932,7 +932,6 @@ int attention_launch(const AttnParams& p, int mode, cudaStream_t st) {
   return f8 ? launch_one<256, 0, 1, true>(p, st) : launch_one<256, 0, 1, false>(p, st);
 }
 
-unsigned int attention_read_status(bool clear) { return read_status_tu(clear); }
-void attention_read_status_async(unsigned int* dst, cudaStream_t st) { read_status_tu_async(dst, st); }
+unsigned int* attention_status_word() { return status_word_tu(); }
 
 }  // namespace oc

@@ -2,6 +2,8 @@
 // can assume alignment and layout; every function launches on the current CUDA stream of the tensor's device.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <mutex>
+
 #include <torch/extension.h>
 
 #include "comm.h"
@@ -1272,33 +1274,37 @@ torch::Tensor sigmoid_mul(torch::Tensor x, torch::Tensor gate) {
   return y;
 }
 
-// Enqueues one small copy per translation unit's status word into `pinned` (int32, >= 16 entries, pinned host memory) on the current
-// stream; the caller reads them after an event recorded behind this call (async scheduling: no device-wide synchronisation).
-void read_status_async(torch::Tensor pinned) {
-  TORCH_CHECK(pinned.scalar_type() == torch::kInt32 && pinned.numel() >= 16 && !pinned.is_cuda() && pinned.is_pinned(), "need 16 pinned int32 words");
-  unsigned int* p = reinterpret_cast<unsigned int*>(pinned.data_ptr<int>());
-  auto st = cur_stream();
-  oc::attention_read_status_async(p + 0, st);
-  oc::attention_tc_read_status_async(p + 1, st);
-  oc::comm_read_status_async(p + 2, st);
-  oc::elementwise_read_status_async(p + 3, st);
-  oc::ep_read_status_async(p + 4, st);
-  oc::gdn_read_status_async(p + 5, st);
-  oc::gemm_read_status_async(p + 6, st);
-  oc::mla_read_status_async(p + 7, st);
-  oc::moe_read_status_async(p + 8, st);
-  oc::sampling_read_status_async(p + 9, st);
-  oc::mla_prefill_read_status_async(p + 10, st);
-  oc::diff_prefill_read_status_async(p + 11, st);
-  oc::talk_prefill_read_status_async(p + 12, st);
-  oc::mla_decode_tc_read_status_async(p + 13, st);
-  oc::gemm_pair_read_status_async(p + 14, st);
+// Addresses of the translation units' status words on the current device.
+static const oc::StatusWords& status_words() {
+  static std::mutex m;
+  static oc::StatusWords words[64] = {};
+  std::lock_guard<std::mutex> lock(m);
+  const int dev = c10::cuda::current_device();
+  TORCH_CHECK(dev >= 0 && dev < 64, "device index");
+  oc::StatusWords& w = words[dev];
+  if (w.n == 0) {
+    oc::StatusWords t{};
+    for (auto get : {oc::attention_status_word, oc::attention_tc_status_word, oc::comm_status_word, oc::elementwise_status_word, oc::ep_status_word,
+                     oc::gdn_status_word, oc::gemm_status_word, oc::mla_status_word, oc::moe_status_word, oc::sampling_status_word,
+                     oc::mla_prefill_status_word, oc::diff_prefill_status_word, oc::talk_prefill_status_word, oc::mla_decode_tc_status_word,
+                     oc::gemm_pair_status_word}) {
+      unsigned int* p = get();
+      TORCH_CHECK(p != nullptr, "a status word has no address");
+      t.w[t.n++] = p;
+    }
+    w = t;
+  }
+  return w;
 }
 
-int64_t read_status(bool clear) {
-  return (int64_t)(oc::gemm_read_status(clear) | oc::gemm_pair_read_status(clear) | oc::elementwise_read_status(clear) | oc::attention_read_status(clear) | oc::attention_tc_read_status(clear) |
-                   oc::comm_read_status(clear) | oc::gdn_read_status(clear) | oc::sampling_read_status(clear) | oc::moe_read_status(clear) | oc::mla_read_status(clear) | oc::mla_decode_tc_read_status(clear) | oc::mla_prefill_read_status(clear) | oc::diff_prefill_read_status(clear) | oc::talk_prefill_read_status(clear) | oc::ep_read_status(clear));
+// Enqueues one kernel that writes every status word into `pinned` (int32, >= 16 entries, pinned host memory) on the current stream; the
+// caller reads them after an event recorded behind this call (async scheduling: no device-wide synchronisation).
+void read_status_async(torch::Tensor pinned) {
+  TORCH_CHECK(pinned.scalar_type() == torch::kInt32 && pinned.numel() >= 16 && !pinned.is_cuda() && pinned.is_pinned(), "need 16 pinned int32 words");
+  TORCH_CHECK(oc::status_gather_launch(status_words(), reinterpret_cast<unsigned int*>(pinned.data_ptr<int>()), cur_stream()) == 0, "status gather failed");
 }
+
+int64_t read_status(bool clear) { return (int64_t)oc::status_read(status_words(), clear); }
 
 // ---- symmetric slab + peer-memory reductions
 int64_t comm_alloc(int64_t bytes) {

@@ -13,7 +13,7 @@ namespace oc {
 // ---- status word -------------------------------------------------------------------------------------------
 // Every bounded wait that gives up ORs a code into this device word instead of trapping; the host reads it
 // after the step. Bits: 0x1 mbarrier wait expired in a GEMM, 0x2 peer-flag wait expired, 0x4 attention, 0x8 other.
-static __device__ unsigned int g_status = 0;  // one per translation unit; each .cu exports a reader
+static __device__ unsigned int g_status = 0;  // one per translation unit; each .cu exports its address (see status.cu)
 enum : unsigned { ST_MBAR_TIMEOUT = 1u, ST_PEER_TIMEOUT = 2u, ST_ATTN = 4u, ST_OTHER = 8u, ST_BOUNDS = 16u };
 
 __device__ __forceinline__ uint64_t globaltimer_ns() {
@@ -322,21 +322,10 @@ static inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 blo
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// Host-side reader for this translation unit's status word.
-static inline unsigned int read_status_tu(bool clear) {
-  unsigned int v = 0;
-  if (cudaMemcpyFromSymbol(&v, g_status, sizeof(v)) != cudaSuccess) return 0x80000000u;
-  if (clear && v) {
-    unsigned int z = 0;
-    cudaMemcpyToSymbol(g_status, &z, sizeof(z));
-  }
-  return v;
-}
-
-// Non-blocking variant: the word lands in (pinned) host memory once the stream reaches the copy, so a step that is still running
-// is not waited for.
-static inline void read_status_tu_async(unsigned int* dst, cudaStream_t st) {
-  cudaMemcpyFromSymbolAsync(dst, g_status, sizeof(unsigned int), 0, cudaMemcpyDeviceToHost, st);
+// Device address of this translation unit's status word on the current device (null when the runtime has none to give).
+static inline unsigned int* status_word_tu() {
+  void* p = nullptr;
+  return cudaGetSymbolAddress(&p, g_status) == cudaSuccess ? static_cast<unsigned int*>(p) : nullptr;
 }
 
 }  // namespace oc

@@ -441,7 +441,6 @@ int diff_prefill_tc_launch(const AttnParams& p, long long num_blocks, cudaStream
   return p.D == 64 ? go<64>(p, num_blocks, st) : go<128>(p, num_blocks, st);
 }
 
-unsigned int diff_prefill_read_status(bool clear) { return read_status_tu(clear); }
-void diff_prefill_read_status_async(unsigned int* dst, cudaStream_t st) { read_status_tu_async(dst, st); }
+unsigned int* diff_prefill_status_word() { return status_word_tu(); }
 
 }  // namespace oc

@@ -469,7 +469,6 @@ int argmax_launch(const void* x, int is_fp32, long long* out, unsigned long long
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-unsigned int elementwise_read_status(bool clear) { return read_status_tu(clear); }
-void elementwise_read_status_async(unsigned int* dst, cudaStream_t st) { read_status_tu_async(dst, st); }
+unsigned int* elementwise_status_word() { return status_word_tu(); }
 
 }  // namespace oc

@@ -236,7 +236,6 @@ int ep_combine_launch(const EpParams& p, const float* w, void* y, int sms, cudaS
   if (p.gather) ep_wait_kernel<<<1, 32, 0, st>>>(p, 3);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
-unsigned int ep_read_status(bool clear) { return read_status_tu(clear); }
-void ep_read_status_async(unsigned int* dst, cudaStream_t st) { read_status_tu_async(dst, st); }
+unsigned int* ep_status_word() { return status_word_tu(); }
 
 }  // namespace oc

@@ -288,7 +288,6 @@ int gdn_recurrent_launch(const GdnParams& p, cudaStream_t st) {
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-unsigned int gdn_read_status(bool clear) { return read_status_tu(clear); }
-void gdn_read_status_async(unsigned int* dst, cudaStream_t st) { read_status_tu_async(dst, st); }
+unsigned int* gdn_status_word() { return status_word_tu(); }
 
 }  // namespace oc

@@ -415,7 +415,6 @@ int gemm_widen_launch(const GemmParams& p, const void* x, int ldx, void* slab, i
   return 0;
 }
 
-unsigned int gemm_pair_read_status(bool clear) { return read_status_tu(clear); }
-void gemm_pair_read_status_async(unsigned int* dst, cudaStream_t st) { read_status_tu_async(dst, st); }
+unsigned int* gemm_pair_status_word() { return status_word_tu(); }
 
 }  // namespace oc

@@ -64,13 +64,11 @@ int gemm_pair_launch(const GemmParams& p, const void* x, int ldx, const void* w,
 bool gemm_widen_takes(const GemmParams& p, int num_sms);
 int gemm_widen_rows(const GemmParams& p, int num_sms);
 int gemm_widen_launch(const GemmParams& p, const void* x, int ldx, void* slab, int num_sms, cudaStream_t st);
-unsigned int gemm_pair_read_status(bool clear);
-void gemm_pair_read_status_async(unsigned int* dst, cudaStream_t st);
+unsigned int* gemm_pair_status_word();
 // a few tokens, packed weights (gemm_skinny.cu)
 bool gemm_skinny_takes(const GemmParams& p);
 int gemm_skinny_launch(const GemmParams& p, const void* x, int ldx, int num_sms, cudaStream_t stream);
-unsigned int gemm_read_status(bool clear);
-void gemm_read_status_async(unsigned int* dst, cudaStream_t st);
+unsigned int* gemm_status_word();
 int gemm_kernel_info(int wkind, int small, int smem, int out[6]);
 
 }  // namespace oc

@@ -6,6 +6,14 @@
 
 namespace oc {
 
+// The translation units' status words (common.cuh), read together (status.cu).
+struct StatusWords {
+  unsigned int* w[16];
+  int n;
+};
+int status_gather_launch(const StatusWords& s, unsigned int* pinned, cudaStream_t st);   // word i -> pinned[i]
+unsigned int status_read(const StatusWords& s, bool clear);                              // all of them, ORed; waits for the device's default stream
+
 struct RopeCacheParams {
   __nv_bfloat16 *q, *k, *v;
   long long q_st, q_sh, k_st, v_st;  // element strides: token / head (k and v heads are D apart)
@@ -81,8 +89,7 @@ int gelu_tanh_f32_launch(float* x, long long n, cudaStream_t st);  // in place
 int argmax_launch(const void* x, int is_fp32, long long* out, unsigned long long* packed, int B, int V, long long ld, cudaStream_t st);
 int merge_attn_states_launch(const void* o1, const float* lse1, const void* o2, const float* lse2, void* out, float* lse_out, int rows, int D,
                              cudaStream_t st);
-unsigned int elementwise_read_status(bool clear);
-void elementwise_read_status_async(unsigned int* dst, cudaStream_t st);
+unsigned int* elementwise_status_word();
 
 struct AttnParams {
   const __nv_bfloat16* q;     // [T][Hq][D] with strides
@@ -130,8 +137,7 @@ int attention_f32_launch(const AttnParams& p, bool bf16, cudaStream_t st);
 // (decode and short verify queries, with split-KV + combine).
 int attention_launch(const AttnParams& p, int mode, cudaStream_t st);
 int attention_decode_fp8_launch(const AttnParams& p, cudaStream_t st);   // its decode mode over an fp8 cache, heads of 128 and 256
-unsigned int attention_read_status(bool clear);
-void attention_read_status_async(unsigned int* dst, cudaStream_t st);
+unsigned int* attention_status_word();
 // Differential attention ahead of its kernels: per (token, head, map) RMS norm and rotation of queries and keys, cache insert.
 struct DiffPrepareParams {
   const void* x;              // [T][ld]: q [2 H dim] | k [2 G dim] | v [G vdim]
@@ -149,13 +155,11 @@ int diff_prepare_launch(const DiffPrepareParams& p, cudaStream_t st);
 // 128-token tiles; q contiguous.
 bool diff_prefill_tc_sizes(int D, float softcap);
 int diff_prefill_tc_launch(const AttnParams& p, long long num_blocks, cudaStream_t st);
-unsigned int diff_prefill_read_status(bool clear);
-void diff_prefill_read_status_async(unsigned int* dst, cudaStream_t st);
+unsigned int* diff_prefill_status_word();
 
 // tcgen05 prefill (attention_tc.cu): D == 128, 128-token query tiles; num_q_tiles counts those tiles.
 int attention_prefill_tc_launch(const AttnParams& p, long long num_blocks, cudaStream_t st);
-unsigned int attention_tc_read_status(bool clear);
-void attention_tc_read_status_async(unsigned int* dst, cudaStream_t st);
+unsigned int* attention_tc_status_word();
 
 
 struct RowStats {
@@ -194,8 +198,7 @@ struct RouteParams {
   float scaling;
 };
 int route_launch(const RouteParams& p, cudaStream_t st);
-unsigned int sampling_read_status(bool clear);
-void sampling_read_status_async(unsigned int* dst, cudaStream_t st);
+unsigned int* sampling_status_word();
 
 struct MoePlanParams {
   int* counts;        // [E] scratch
@@ -215,8 +218,7 @@ int moe_gemm_f32_launch(const float* x, int ldx, const float* w, float* out, int
                         int num_sms, cudaStream_t st);
 int moe_plan_launch(const MoePlanParams& p, cudaStream_t st);
 int moe_combine_launch(const void* a2, int lda, const int* slot_of, const float* w, void* y, int T, int k, int H, int f32, cudaStream_t st);
-unsigned int moe_read_status(bool clear);
-void moe_read_status_async(unsigned int* dst, cudaStream_t st);
+unsigned int* moe_status_word();
 
 struct MlaParams {
   const void* q_abs;            // [T][H][kv_lora] query with W_UK absorbed, contiguous
@@ -243,8 +245,7 @@ struct MlaParams {
 };
 bool mla_decode_tc_takes(int kv_lora, int rope_pad, int bs, int fine, float scale);
 int mla_decode_tc_launch(const MlaParams& p, cudaStream_t st);
-unsigned int mla_decode_tc_read_status(bool clear);
-void mla_decode_tc_read_status_async(unsigned int* dst, cudaStream_t st);
+unsigned int* mla_decode_tc_status_word();
 int mla_decode_launch(const MlaParams& p, cudaStream_t st);
 bool mla_tensor_core_sizes(int kv_lora, int rope_pad);
 // Prefill in the expanded form: gathered latents -> per-head keys and values (a GEMM in between) -> causal attention.
@@ -268,8 +269,7 @@ struct MlaPrefillParams {
 bool mla_prefill_sizes(int nope, int rope, int vd);
 int mla_prefill_inputs_launch(const MlaPrefillParams& p, cudaStream_t st);   // gather + query rows
 int mla_prefill_launch(const MlaPrefillParams& p, cudaStream_t st);
-unsigned int mla_prefill_read_status(bool clear);
-void mla_prefill_read_status_async(unsigned int* dst, cudaStream_t st);
+unsigned int* mla_prefill_status_word();
 struct MlaPrepareParams {
   const void *q, *kv;           // query latent [T][nq] or null; [T][lora + rope], pitches ld_q / ld_kv
   long long ld_q, ld_kv;
@@ -306,8 +306,7 @@ int mlstm_recurrent_launch(const MlstmParams& p, cudaStream_t st);
 bool mlstm_chunkable(int D, int V);
 int mlstm_chunk_launch(const MlstmParams& p, int num_chunks, int num_long, cudaStream_t st);
 int sigmoid_mul_launch(const void* x, long long ldx, const void* gate, long long ldg, void* y, int T, int N, int f32, cudaStream_t st);
-unsigned int mla_read_status(bool clear);
-void mla_read_status_async(unsigned int* dst, cudaStream_t st);
+unsigned int* mla_status_word();
 
 struct GdnConvParams {
   const __nv_bfloat16* x;   // [T][ldx] pre-conv mixed q|k|v (column slice allowed)
@@ -369,8 +368,7 @@ int gdn_chunk_launch(const GdnChunkParams& p, cudaStream_t st);
 int gdn_conv_launch(const GdnConvParams& p, cudaStream_t st);
 int gdn_conv_commit_launch(const GdnConvParams& p, cudaStream_t st);
 int gdn_recurrent_launch(const GdnParams& p, cudaStream_t st);
-unsigned int gdn_read_status(bool clear);
-void gdn_read_status_async(unsigned int* dst, cudaStream_t st);
+unsigned int* gdn_status_word();
 
 struct CausalConvParams {
   const void* x;                // [T][C], row pitch ldx
@@ -463,7 +461,6 @@ int talk_decode_launch(const TalkTcParams& p, cudaStream_t st);
 int talk_join_launch(const TalkTcParams& p, bool dec, int rows, cudaStream_t st);
 // tiles: 128-token tiles over the portions; `segment` of them at a time go through the workspace
 int talk_prefill_launch(const TalkTcParams& p, int tiles, int segment, long long num_blocks, cudaStream_t st);
-unsigned int talk_prefill_read_status(bool clear);
-void talk_prefill_read_status_async(unsigned int* dst, cudaStream_t st);
+unsigned int* talk_prefill_status_word();
 
 }  // namespace oc

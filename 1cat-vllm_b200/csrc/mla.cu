@@ -496,7 +496,6 @@ int mla_prepare_launch(const MlaPrepareParams& p, cudaStream_t st) {
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
-unsigned int mla_read_status(bool clear) { return read_status_tu(clear); }
-void mla_read_status_async(unsigned int* dst, cudaStream_t st) { read_status_tu_async(dst, st); }
+unsigned int* mla_status_word() { return status_word_tu(); }
 
 }  // namespace oc

@@ -448,7 +448,6 @@ int mla_decode_tc_launch(const MlaParams& p, cudaStream_t st) {
   return launch_k(mla_decode_tc_kernel, grid, dim3(kThreads), (size_t)kSmem, st, true, tmQ, tmK, p) == cudaSuccess ? 0 : -5;
 }
 
-unsigned int mla_decode_tc_read_status(bool clear) { return read_status_tu(clear); }
-void mla_decode_tc_read_status_async(unsigned int* dst, cudaStream_t st) { read_status_tu_async(dst, st); }
+unsigned int* mla_decode_tc_status_word() { return status_word_tu(); }
 
 }  // namespace oc

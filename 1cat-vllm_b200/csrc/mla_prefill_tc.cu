@@ -461,7 +461,6 @@ int mla_prefill_launch(const MlaPrefillParams& p, cudaStream_t st) {
   return VC == 1 ? go_fine<3, 1>(p, st) : go_fine<3, 2>(p, st);
 }
 
-unsigned int mla_prefill_read_status(bool clear) { return read_status_tu(clear); }
-void mla_prefill_read_status_async(unsigned int* dst, cudaStream_t st) { read_status_tu_async(dst, st); }
+unsigned int* mla_prefill_status_word() { return status_word_tu(); }
 
 }  // namespace oc

@@ -224,7 +224,6 @@ int moe_combine_launch(const void* a2, int lda, const int* slot_of, const float*
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-unsigned int moe_read_status(bool clear) { return read_status_tu(clear); }
-void moe_read_status_async(unsigned int* dst, cudaStream_t st) { read_status_tu_async(dst, st); }
+unsigned int* moe_status_word() { return status_word_tu(); }
 
 }  // namespace oc

@@ -234,7 +234,6 @@ int route_launch(const RouteParams& q, cudaStream_t st) {
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-unsigned int sampling_read_status(bool clear) { return read_status_tu(clear); }
-void sampling_read_status_async(unsigned int* dst, cudaStream_t st) { read_status_tu_async(dst, st); }
+unsigned int* sampling_status_word() { return status_word_tu(); }
 
 }  // namespace oc

@@ -502,7 +502,6 @@ int talk_prefill_launch(const TalkTcParams& p_, int tiles, int segment, long lon
   return p.t.row == 64 ? go<1>(p, tiles, segment, num_blocks, st) : go<2>(p, tiles, segment, num_blocks, st);
 }
 
-unsigned int talk_prefill_read_status(bool clear) { return read_status_tu(clear); }
-void talk_prefill_read_status_async(unsigned int* dst, cudaStream_t st) { read_status_tu_async(dst, st); }
+unsigned int* talk_prefill_status_word() { return status_word_tu(); }
 
 }  // namespace oc
