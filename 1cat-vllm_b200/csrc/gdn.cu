@@ -88,6 +88,61 @@ __global__ void gdn_conv_kernel(const GdnConvParams p) {
   }
 }
 
+// The same for eight tokens and eight channels per thread (4 taps): the eleven input rows are read once instead of once per tap, all in flight together,
+// and the taps are widened once. Sums in the same order. For steps of many tokens: a decoding step has too few for it. Bound by memory, a
+// step's channels once in and once out: 3950 tokens x 10240 channels 53 us
+// where a thread per token took 87.
+constexpr int kConvTokens = 8;
+__global__ void __launch_bounds__(128) gdn_conv_tile_kernel(const GdnConvParams p) {
+  const int c = (blockIdx.x * 128 + threadIdx.x) * 8, tb = blockIdx.y * kConvTokens;
+  __shared__ int s_t0[kConvTokens], s_r[kConvTokens];
+  if (threadIdx.x < kConvTokens) {
+    const int r = find_request(p.query_start_loc, p.R, min(tb + (int)threadIdx.x, p.T - 1));
+    s_r[threadIdx.x] = r;
+    s_t0[threadIdx.x] = p.query_start_loc[r];
+  }
+  __syncthreads();
+  if (c >= p.C) return;
+  uint4 row[kConvTokens + 3];             // inputs of tokens tb - 3 .. tb + 7
+#pragma unroll
+  for (int i = 0; i < kConvTokens + 3; ++i) {
+    const int t = tb - 3 + i;
+    row[i] = t >= 0 && t < p.T ? *reinterpret_cast<const uint4*>(p.x + (size_t)t * p.ldx + c) : make_uint4(0, 0, 0, 0);
+  }
+  float wv[8][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint4 raw = reinterpret_cast<const uint4*>(p.w + (size_t)c * 4)[i];
+    const __nv_bfloat16* rp = reinterpret_cast<const __nv_bfloat16*>(&raw);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) wv[(i * 8 + e) >> 2][(i * 8 + e) & 3] = __bfloat162float(rp[e]);
+  }
+#pragma unroll
+  for (int i = 0; i < kConvTokens; ++i) {
+    const int t = tb + i;
+    if (t >= p.T) break;
+    const int pos = t - s_t0[i];          // position in the sequence's new tokens
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (pos - 3 + j >= 0) {
+        const __nv_bfloat16* rp = reinterpret_cast<const __nv_bfloat16*>(&row[i + j]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += __bfloat162float(rp[e]) * wv[e][j];
+      } else if (p.has_initial_state[s_r[i]] != 0) {
+        const __nv_bfloat16* st = p.conv_state + ((size_t)p.state_slots[s_r[i]] * p.C + c) * 3 + pos + j;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += __bfloat162float(st[e * 3]) * wv[e][j];
+      }
+    }
+    uint4 o;
+    __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(&o);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) op[e] = __float2bfloat16(acc[e] / (1.f + __expf(-acc[e])));
+    *reinterpret_cast<uint4*>(p.y + (size_t)t * p.C + c) = o;
+  }
+}
+
 // conv_state[slot][c][:] <- the last kw-1 inputs of the sequence (mixing old state and new tokens when the chunk is short).
 // Must run after gdn_conv_kernel (it overwrites what that kernel reads). One thread per (request, channel).
 __global__ void gdn_conv_state_kernel(const GdnConvParams p) {
@@ -262,8 +317,9 @@ int gdn_conv_launch(const GdnConvParams& p, cudaStream_t st) {
   if (p.T == 0) return 0;
   if (p.kw < 2 || p.kw > 8) return -1;
   if (p.kw == 4 && p.C % 8 == 0 && p.ldx % 8 == 0 && ((uintptr_t)p.x & 15) == 0 && ((uintptr_t)p.y & 15) == 0 && ((uintptr_t)p.w & 15) == 0) {
-    dim3 grid((p.C / 8 + 127) / 128, p.T);
-    gdn_conv_kernel<8><<<grid, 128, 0, st>>>(p);
+    const unsigned gx = (unsigned)((p.C / 8 + 127) / 128);
+    if (p.T >= 512) gdn_conv_tile_kernel<<<dim3(gx, (p.T + kConvTokens - 1) / kConvTokens), 128, 0, st>>>(p);
+    else gdn_conv_kernel<8><<<dim3(gx, p.T), 128, 0, st>>>(p);
   } else {
     dim3 grid((p.C + 255) / 256, p.T);
     gdn_conv_kernel<1><<<grid, 256, 0, st>>>(p);

@@ -230,3 +230,26 @@ def test_packed_gemm_of_many_tokens(kind, T, N, Kd, gated):
     torch.cuda.synchronize()
     assert K().check_status() == 0 and (out[T:] == 7).all() and (out[:, want.shape[1]:] == 7).all()
     _close(out[:T, : want.shape[1]], want, 2 ** -6, float(want.abs().mean()) * 2 ** -6, f"kind {kind}")
+
+
+@pytest.mark.parametrize("qlens,fresh", [([1, 2, 3, 500, 5, 1], [0, 0, 1, 1, 0, 1]), ([515], [1]), ([300, 4, 1, 210], [0, 1, 0, 0])])
+def test_causal_convolution_of_eight_tokens_a_thread(qlens, fresh):
+    """Sequences that begin and end inside a tile of eight tokens, shorter than the taps, with and without a state, through the recurrent layer's step (its
+    other kernels have tests of their own). Tolerances as there: bf16 products of normalised keys along the sequence."""
+    from onecat_vllm.worker.attn_metadata import AttentionMetadata
+    Hk, Hv, D, R, T = 1, 1, 128, len(qlens), sum(qlens)
+    C = (2 * Hk + Hv) * D
+    g = torch.Generator().manual_seed(T)
+    x, w = (torch.randn(T, C, generator=g) * 0.5).bfloat16(), (torch.randn(C, 4, generator=g) * 0.3).bfloat16()
+    ba, A_log, dt = torch.randn(T, 2 * Hv, generator=g).bfloat16(), torch.rand(Hv, generator=g) - 1.0, torch.rand(Hv, generator=g)
+    conv, state = (torch.randn(R + 1, C, 3, generator=g) * 0.5).bfloat16(), torch.randn(R + 1, Hv, D, D, generator=g) * 0.1
+    qsl = torch.tensor([0, *torch.tensor(qlens).cumsum(0).tolist()], dtype=torch.int32)
+    slots, has = torch.randperm(R + 1, generator=g)[:R].to(torch.int32), 1 - torch.tensor(fresh, dtype=torch.int32)
+    md = AttentionMetadata(R, T, qsl.cuda(), None, None, None, None, max(qlens), 0, state_slots=slots.cuda(), has_initial_state=has.cuda(), query_lens_cpu=list(qlens))
+    dconv, dstate, dba = conv.cuda(), state.cuda(), ba.cuda()
+    out = K().gdn_forward(x.cuda(), dba[:, :Hv], dba[:, Hv:], w.cuda(), A_log.cuda(), dt.cuda(), dconv, dstate, md, Hk, Hv, D, D)
+    m = ref.causal_conv1d(x, w, None, conv, qsl, slots, has)
+    gate, beta = ref.gdn_gating(ba[:, Hv:], ba[:, :Hv], A_log, dt)
+    want = ref.gated_delta_rule(m[:, :D].reshape(T, 1, D), m[:, D:2 * D].reshape(T, 1, D), m[:, 2 * D:].reshape(T, 1, D), gate, beta, state, qsl, slots, has)
+    _close(out.view(T, Hv, D), want, 4e-2, 4e-2)
+    assert torch.equal(dconv.cpu(), conv)
