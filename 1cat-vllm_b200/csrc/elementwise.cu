@@ -108,6 +108,49 @@ __global__ void rms_norm_gated_kernel(const __nv_bfloat16* __restrict__ x, const
   }
 }
 
+// The same in 16-byte accesses, a group of D / 8 lanes per row and two rows per group: bound by memory (x and z in, y out), 3950 tokens x 48 heads of
+// 128 23 us where two-byte accesses took 54.
+template <int D>
+__global__ void __launch_bounds__(256) rms_norm_gated_vec_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ z,
+                                                                 const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, int rows, int ldx, int ldz,
+                                                                 int heads, float eps) {
+  constexpr int LPH = D / 8, U = 2;
+  const int sub = threadIdx.x % LPH, row0 = (blockIdx.x * (256 / LPH) + threadIdx.x / LPH) * U;
+  uint4 xv[U], zv[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    xv[u] = zv[u] = make_uint4(0, 0, 0, 0);
+    if (row0 + u < rows) {                // every lane stays for the shuffles
+      const size_t tok = (row0 + u) / heads, at = (size_t)((row0 + u) % heads) * D + sub * 8;
+      xv[u] = *reinterpret_cast<const uint4*>(x + tok * ldx + at);
+      zv[u] = *reinterpret_cast<const uint4*>(z + tok * ldz + at);
+    }
+  }
+  const uint4 wr = *reinterpret_cast<const uint4*>(w + sub * 8);
+  const __nv_bfloat16* wp = reinterpret_cast<const __nv_bfloat16*>(&wr);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const __nv_bfloat16 *xp = reinterpret_cast<const __nv_bfloat16*>(&xv[u]), *zp = reinterpret_cast<const __nv_bfloat16*>(&zv[u]);
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float v = __bfloat162float(xp[i]);
+      ss += v * v;
+    }
+#pragma unroll
+    for (int o = LPH / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float inv = rsqrtf(ss / (float)D + eps);
+    uint4 out;
+    __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(&out);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float g = __bfloat162float(zp[i]);
+      op[i] = __float2bfloat16(__bfloat162float(xp[i]) * inv * __bfloat162float(wp[i]) * (g / (1.f + __expf(-g))));
+    }
+    if (row0 + u < rows) *reinterpret_cast<uint4*>(y + (size_t)(row0 + u) * D + sub * 8) = out;
+  }
+}
+
 __global__ void silu_and_mul_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, int T, int I) {
   size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   size_t total = (size_t)T * I / 8;
@@ -390,6 +433,16 @@ int rms_norm_gated_launch(const void* x, const void* z, const void* w, void* y, 
                           float eps, cudaStream_t st) {
   if (D % 32 || D > 256) return -1;
   if (rows == 0) return 0;
+  auto al = [](const void* v) { return ((uintptr_t)v & 15) == 0; };
+  if ((D == 64 || D == 128 || D == 256) && ldx % 8 == 0 && ldz % 8 == 0 && al(x) && al(z) && al(w) && al(y)) {
+    auto go = [&](auto kernel) {
+      const int per = 256 / (D / 8) * 2;
+      kernel<<<(rows + per - 1) / per, 256, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)z, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, rows, ldx, ldz,
+                                                     heads, eps);
+      return cudaGetLastError() == cudaSuccess ? 0 : -2;
+    };
+    return D == 64 ? go(rms_norm_gated_vec_kernel<64>) : D == 128 ? go(rms_norm_gated_vec_kernel<128>) : go(rms_norm_gated_vec_kernel<256>);
+  }
   rms_norm_gated_kernel<<<(rows + 7) / 8, 256, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)z, (const __nv_bfloat16*)w,
                                                         (__nv_bfloat16*)y, rows, D, ldx, ldz, heads, eps);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;

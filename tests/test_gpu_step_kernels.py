@@ -253,3 +253,13 @@ def test_causal_convolution_of_eight_tokens_a_thread(qlens, fresh):
     want = ref.gated_delta_rule(m[:, :D].reshape(T, 1, D), m[:, D:2 * D].reshape(T, 1, D), m[:, 2 * D:].reshape(T, 1, D), gate, beta, state, qsl, slots, has)
     _close(out.view(T, Hv, D), want, 4e-2, 4e-2)
     assert torch.equal(dconv.cpu(), conv)
+
+
+@pytest.mark.parametrize("T,heads,D", [(1, 1, 64), (7, 3, 128), (33, 5, 256), (130, 48, 128)])
+def test_gated_norm_in_wide_accesses(T, heads, D):
+    """Odd numbers of rows (a group takes two), slices of wider rows; one rounding of fp32 arithmetic."""
+    g = torch.Generator().manual_seed(T)
+    x, wide, w = torch.randn(T, heads * D, generator=g).bfloat16(), torch.randn(T, 2 * heads * D, generator=g).bfloat16(), (1 + 0.1 * torch.randn(D, generator=g)).bfloat16()
+    z = wide[:, heads * D:]
+    y = K().rms_norm_gated(x.cuda(), wide.cuda()[:, heads * D:], w.cuda(), 1e-6, heads)
+    _close(y.view(T, heads, D), ref.rms_norm_gated(x.view(T, heads, D), z.reshape(T, heads, D), w, 1e-6), 2 ** -6, 2 ** -8)
