@@ -917,6 +917,7 @@ torch::Tensor mla_decode(torch::Tensor q_abs, torch::Tensor q_rope, torch::Tenso
   p.bt_stride = (int)block_table.stride(0); p.R = (int)seq_lens.size(0);
   p.bs = (int)cache.size(1); p.bs_shift = 0;
   p.num_blocks = (int)cache.size(0);
+  p.halves = 1;
   while ((1 << p.bs_shift) < p.bs) ++p.bs_shift;
   p.max_q_len = (int)max_q_len; p.splits = (int)splits; p.scale = (float)scale;
   check_sink_gate(sinks, gate, et, p.T, p.H);
@@ -924,7 +925,7 @@ torch::Tensor mla_decode(torch::Tensor q_abs, torch::Tensor q_rope, torch::Tenso
   if (gate.has_value()) { p.gate = gate->data_ptr(); p.gate_st = gate->stride(0); }
   if (splits > 1) {
     TORCH_CHECK(ws_o.has_value() && ws_ml.has_value() && (size_t)ws_o->numel() >= (size_t)splits * p.T * p.H * p.kv_lora &&
-                (size_t)ws_ml->numel() >= (size_t)splits * p.T * p.H * 2, "split-KV workspace too small");
+                (size_t)ws_ml->numel() >= (size_t)splits * p.T * p.H * 4, "split-KV workspace too small");   // a reference and a sum for each half of the columns
     p.ws_o = ws_o->data_ptr<float>(); p.ws_ml = ws_ml->data_ptr<float>();
   }
   int rc = oc::mla_decode_launch(p, cur_stream());

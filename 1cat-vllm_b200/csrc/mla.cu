@@ -264,29 +264,35 @@ __global__ void mla_combine_kernel(const MlaParams p) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, DV = p.kv_lora;
   const int rows = p.T * p.H;
   if (warp >= rows) return;
-  float mine = lane < p.splits ? p.ws_ml[((size_t)lane * rows + warp) * 2] : -INFINITY;   // at most 32 splits
-  const float M = warp_max(mine);
-  const float f_mine = mine == -INFINITY ? 0.f : ex2(mine - M);
-  const float L = warp_sum(lane < p.splits ? p.ws_ml[((size_t)lane * rows + warp) * 2 + 1] * f_mine : 0.f);
-  const float den = L + (p.sinks != nullptr ? ex2(p.sinks[warp % p.H] * 1.4426950408889634f - M) : 0.f);
-  const float inv = L > 0.f ? gate_of<__nv_bfloat16>(p, warp / p.H, warp % p.H) / den : 0.f;
-  // 16-byte loads, four splits of a column block in flight
-  for (int c = lane * 4; c < (DV + 127) / 128 * 128; c += 128) {
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s0 = 0; s0 < p.splits; s0 += 4) {
-      float4 v[4];
-      float f[4];
+  // mla_decode_tc.cu: the two halves of the columns come from CTAs with references of their own
+  for (int h = 0; h < p.halves; ++h) {
+    const float* ml = p.ws_ml + (((size_t)lane * rows + warp) * p.halves + h) * 2;
+    const float mine = lane < p.splits ? ml[0] : -INFINITY;   // at most 32 splits
+    const float M = warp_max(mine);
+    const float f_mine = mine == -INFINITY ? 0.f : ex2(mine - M);
+    const float L = warp_sum(lane < p.splits ? ml[1] * f_mine : 0.f);
+    const float den = L + (p.sinks != nullptr ? ex2(p.sinks[warp % p.H] * 1.4426950408889634f - M) : 0.f);
+    const float inv = L > 0.f ? gate_of<__nv_bfloat16>(p, warp / p.H, warp % p.H) / den : 0.f;
+    const int c1 = (h + 1) * (DV / p.halves);
+    // 16-byte loads, four splits of a column block in flight
+    for (int c0 = h * (DV / p.halves); c0 < c1; c0 += 128) {
+      const int c = c0 + lane * 4;
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int s0 = 0; s0 < p.splits; s0 += 4) {
+        float4 v[4];
+        float f[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        f[i] = s0 + i < p.splits ? __shfl_sync(0xffffffffu, f_mine, s0 + i) : 0.f;
-        v[i] = f[i] != 0.f && c < DV ? *reinterpret_cast<const float4*>(p.ws_o + ((size_t)(s0 + i) * rows + warp) * DV + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = 0; i < 4; ++i) {
+          f[i] = s0 + i < p.splits ? __shfl_sync(0xffffffffu, f_mine, s0 + i) : 0.f;
+          v[i] = f[i] != 0.f && c < c1 ? *reinterpret_cast<const float4*>(p.ws_o + ((size_t)(s0 + i) * rows + warp) * DV + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (f[i] != 0.f) x = make_float4(fmaf(v[i].x, f[i], x.x), fmaf(v[i].y, f[i], x.y), fmaf(v[i].z, f[i], x.z), fmaf(v[i].w, f[i], x.w));
       }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (f[i] != 0.f) x = make_float4(fmaf(v[i].x, f[i], x.x), fmaf(v[i].y, f[i], x.y), fmaf(v[i].z, f[i], x.z), fmaf(v[i].w, f[i], x.w));
+      if (c < c1)
+        *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)warp * DV + c) = make_uint2(pk(x.x * inv, x.y * inv), pk(x.z * inv, x.w * inv));
     }
-    if (c < DV)
-      *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)warp * DV + c) = make_uint2(pk(x.x * inv, x.y * inv), pk(x.z * inv, x.w * inv));
   }
 }
 
@@ -474,9 +480,11 @@ int mla_decode_launch(const MlaParams& p, cudaStream_t st) {
   if (p.f32) return p.splits == 1 ? plain_e<float>(p, st) : -1;
   if (!mla_tensor_core_sizes(p.kv_lora, p.rope_pad)) return p.splits == 1 ? plain_e<__nv_bfloat16>(p, st) : -1;
   if (mla_decode_tc_takes(p.kv_lora, p.rope_pad, p.bs, p.fine, p.scale)) {
-    const int rc = mla_decode_tc_launch(p, st);
+    MlaParams w = p;
+    w.halves = 2;
+    const int rc = mla_decode_tc_launch(w, st);
     if (rc != 0) return rc;
-    if (p.splits > 1) mla_combine_kernel<<<(p.T * p.H * 32 + 255) / 256, 256, 0, st>>>(p);
+    if (p.splits > 1) mla_combine_kernel<<<(p.T * p.H * 32 + 255) / 256, 256, 0, st>>>(w);
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
   }
   switch (p.kv_lora) {

@@ -7,7 +7,8 @@
 //   P = softmax    four warps, one thread per row; P replaces S in its TMEM columns as bf16
 //   O += P V       operand A from TMEM, V = this CTA's 256 latent columns of the same key tile as an MN-major operand, O [128 x 256] in TMEM
 // Both halves compute all scores (576 + 256 instead of 576 / 2 + 256 products per key): that keeps O in half of the tensor memory, where the
-// whole of it would leave no room for S, and needs no exchange between CTAs. The second CTA's key tiles come from L2.
+// whole of it would leave no room for S, and needs no exchange between CTAs. The second CTA's key tiles come from L2. The two sum a score in
+// different orders, so one may take a new reference where the other keeps its own: each hands its (reference, sum) to the merge of the splits.
 // Operand Q does not fit beside two key tiles (144 of 227 KB), so the 256 columns of it that meet this CTA's value columns live in TMEM, and
 // the other 256 + 64 in shared memory. A key tile (64 keys, 72 KB) is loaded in two groups, each with barriers of its own: group A (the five
 // column chunks only scores need) is free again after the scores, group B (the four chunks that are also values) after the value product.
@@ -100,8 +101,8 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   }
   const int n = hi - lo;                     // tiles of this CTA
   if (n <= 0) {                              // an empty split: a sum of nothing (the merge skips its columns)
-    if (half == 0 && threadIdx.x < nrows) {
-      float* wm = p.ws_ml + ((size_t)split * p.T * p.H + (size_t)qs * p.H + row0 + threadIdx.x) * 2;
+    if (threadIdx.x < nrows) {
+      float* wm = p.ws_ml + (((size_t)split * p.T * p.H + (size_t)qs * p.H + row0 + threadIdx.x) * 2 + half) * 2;
       wm[0] = -INFINITY;
       wm[1] = 0.f;
     }
@@ -381,8 +382,8 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           for (int i = 0; i < 16; i += 4) *reinterpret_cast<uint4*>(dst + c + 2 * i) = make_uint4(w[i], w[i + 1], w[i + 2], w[i + 3]);
         }
       }
-      if (part && half == 0 && live) {
-        float* wm = p.ws_ml + ((size_t)split * p.T * p.H + orow) * 2;
+      if (part && live) {                      // of this half: the other CTA may have another reference
+        float* wm = p.ws_ml + (((size_t)split * p.T * p.H + orow) * 2 + half) * 2;
         wm[0] = m;
         wm[1] = l;
       }

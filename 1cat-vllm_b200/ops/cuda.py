@@ -50,6 +50,7 @@ class _Workspace:
             # a later engine in the same process may need more; graphs captured earlier keep their (retired) buffers alive
             if getattr(self, "s_o", None) is not None:
                 self._retired = getattr(self, "_retired", []) + [(self.s_o, self.s_ml)]
+                n_o, n_ml = max(n_o, self.s_o.numel()), max(n_ml, self.s_ml.numel())   # neither shrinks: layers of several kinds take turns
             self.s_o = torch.empty(n_o, dtype=torch.float32, device=self.device)
             self.s_ml = torch.empty(n_ml, dtype=torch.float32, device=self.device)
         return self.s_o, self.s_ml
@@ -850,7 +851,7 @@ def mla_decode(q_abs, q_pe, latent_cache, md, scale, lora, cos_sin=None, interle
             splits = plan_mla_splits(H, lora, ql, sl, _sms(q_abs.device))
         if splits > 1:
             w = workspace(q_abs.device)
-            ws_o, ws_ml = (w.attn_static if static else w.attn)(splits * T * H * lora, splits * T * H * 2)
+            ws_o, ws_ml = (w.attn_static if static else w.attn)(splits * T * H * lora, splits * T * H * 4)   # a reference and a sum for each half of the columns
     _LAUNCHES += 2 if splits > 1 else 1
     return _C.mla_decode(q_abs, q_pe, latent_cache, md.query_start_loc, md.seq_lens, md.block_table, scale, max(ql), splits, ws_o, ws_ml, cos_sin,
                          interleaved, fine, skip_min_len, sinks, gate)

@@ -51,7 +51,7 @@ class DecodeGraphs:
             self.geom = (a.Hq, a.Hkv, a.D)
             K.workspace(runner.device).attn_static(32 * tmax * max(a.Hq * a.D for a in attns), 32 * tmax * 2 * max(a.Hq for a in attns))
             for a in mlas:
-                K.workspace(runner.device).attn_static(32 * tmax * a.H * a.lora_pad, 32 * tmax * a.H * 2)
+                K.workspace(runner.device).attn_static(32 * tmax * a.H * a.lora_pad, 32 * tmax * a.H * 4)
             for a in attns:
                 if getattr(a, "token_scale", False):
                     K.workspace(runner.device).attn_static(*K.talk_workspace(a.Hq, a.Hkv, a.D, tmax))
@@ -60,7 +60,7 @@ class DecodeGraphs:
         elif mla:
             self.geom = ("mla", mlas[0].H, mlas[0].lora_pad)
             for a in mlas:
-                K.workspace(runner.device).attn_static(32 * tmax * a.H * a.lora_pad, 32 * tmax * a.H * 2)
+                K.workspace(runner.device).attn_static(32 * tmax * a.H * a.lora_pad, 32 * tmax * a.H * 4)
         else:
             self.geom, self.max_span = ("state",), 1   # recurrent layers only: nothing depends on the context length
         # every mixer's decode path runs without host synchronisation on fixed addresses (attention, latent attention, Gated-DeltaNet

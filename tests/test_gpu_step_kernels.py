@@ -76,6 +76,76 @@ def test_mla_decode_tiles_of_128_rows(qlens, ctxs, H, rope, options):
         _close(out, want, 2e-2, 5e-3)
 
 
+def _mla_case(qlens, seq, H, g, q_pe, k_pe, lora=512, rope=64, bs=16):
+    """(queries, rotated queries, cache in shuffled pages, block table, query starts, lengths, metadata): random latents beside given rotated parts."""
+    from onecat_vllm.worker.attn_metadata import AttentionMetadata
+    R, T = len(qlens), sum(qlens)
+    per = [-(-s // bs) for s in seq]
+    order = torch.randperm(sum(per), generator=g).to(torch.int32) + 1
+    bt, at = torch.zeros(R, max(per), dtype=torch.int32), 0
+    cache = (torch.randn(sum(per) + 1, bs, lora + rope, generator=g) * 0.3).bfloat16()
+    for r, n in enumerate(per):
+        bt[r, :n] = order[at:at + n]
+        at += n
+        rows = torch.zeros(n * bs, rope)
+        rows[: seq[r]] = k_pe[r]
+        cache[bt[r, :n].long(), :, lora:] = rows.view(n, bs, rope).bfloat16()
+    q = (torch.randn(T, H, lora, generator=g) * 0.5).bfloat16()
+    qsl, sl = torch.tensor([0, *torch.tensor(qlens).cumsum(0).tolist()], dtype=torch.int32), torch.tensor(seq, dtype=torch.int32)
+    md = AttentionMetadata(R, T, qsl.cuda(), sl.cuda(), bt.cuda(), None, None, max(qlens), max(seq), query_lens_cpu=list(qlens), seq_lens_cpu=seq)
+    return q, q_pe.bfloat16(), cache, bt, qsl, sl, md
+
+
+def _in_splits(md, H, splits):
+    md.static_ws, md.attn_plan = True, (("mla", H, 512), (md.max_query_len, 0, splits))
+    return md
+
+
+@pytest.mark.parametrize("splits", [2, 4])
+def test_mla_decode_halves_of_the_columns_at_the_edge_of_a_new_reference(splits):
+    """The CTAs of the two column halves sum a score in different orders. Where a row's maximum grows by 2^8 to within that difference, one of them
+    may move its reference and the other not: each half is merged by its own. Parts of the scores that cancel widen the difference; the scale
+    puts one head after another on the edge, between the first and the second tile of a split."""
+    H, S, T = 128, 512, 1
+    g = torch.Generator().manual_seed(splits)
+    k_pe, q_pe = torch.zeros(1, S, 64), torch.zeros(T, H, 64)
+    q_pe[..., 0] = 4
+    k_pe[0, S // splits - 30, 0] = k_pe[0, -5, 0] = 10   # raw scores rise by 40, in the last tile of the first and of the last split
+    q, q_pe, cache, bt, qsl, sl, md = _mla_case([1], [S], H, g, q_pe, k_pe)
+    q[..., :32], q[..., 256:288], cache[..., :32], cache[..., 256:288] = 16, -16, 8, 8   # 4096 - 4096
+    _in_splits(md, H, splits)
+    dev = [t.cuda() for t in (q, q_pe, cache)]
+    kv = cache[bt[0].long()].reshape(S, 576).double()
+    raw = torch.cat([q, q_pe], -1)[0].double() @ kv.t()
+    tiles = raw[:, : S // splits].view(H, -1, 64).amax(-1)
+    growth = tiles[:, -1] - tiles[:, :-1].amax(-1)
+    for h in range(0, H, 8):
+        for off in (-1e-4, -3e-5, 0.0, 3e-5, 1e-4):
+            scale = 8 / 1.4426950408889634 / float(growth[h]) * (1 + off)
+            want = torch.softmax(raw * scale, -1) @ kv[:, :512]
+            out = K().mla_decode(*dev, md, scale, 512)
+            _close(out[0], want, 2e-2, 5e-2, f"head {h}, {off}")   # weights in bf16 (2^-8); results of up to 8
+    assert K().check_status() == 0
+
+
+@pytest.mark.parametrize("qlens,ctxs,H,step", [([1, 1], [700, 128], 128, 6.0), ([1, 3, 2], [320, 500, 63], 64, 25.0), ([5], [1000], 16, 60.0), ([1] * 3, [640, 65, 1], 128, -9.0)])
+@pytest.mark.parametrize("splits", [1, 2, 3])
+def test_mla_decode_rescales_its_results(qlens, ctxs, H, step, splits):
+    """Maxima that grow (or fall) from tile to tile by 2^2 to 2^40, differently in every head: the results so far are rescaled in some rows of a warp
+    and tiles, in one split and several, with several tokens a request. Weights and queries are bf16: 2^-8 each."""
+    seq = [c + q for q, c in zip(qlens, ctxs)]
+    g = torch.Generator().manual_seed(sum(seq) + splits)
+    k_pe = [torch.zeros(s, 64) for s in seq]
+    for k in k_pe:
+        k[:, 0] = (torch.arange(len(k)) // 64) * step
+    q_pe = torch.zeros(sum(qlens), H, 64)
+    q_pe[..., 0] = torch.rand(sum(qlens), H, generator=g) * 8
+    q, q_pe, cache, bt, qsl, sl, md = _mla_case(qlens, seq, H, g, q_pe, k_pe)
+    out = K().mla_decode(q.cuda(), q_pe.cuda(), cache.cuda(), _in_splits(md, H, splits), 192 ** -0.5, 512)
+    assert K().check_status() == 0
+    _close(out, ref.mla_decode(q, q_pe, cache, bt, qsl, sl, 192 ** -0.5, 512), 2e-2, 1e-2)
+
+
 def _packed(kind, N, Kd, g):
     """(packed tiles, scale table, padded rows, k tiles per group, weights in fp64) of random weights."""
     n = 64 if Kd % 128 else 128   # group
