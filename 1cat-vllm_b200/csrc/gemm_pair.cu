@@ -113,16 +113,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         int tt, nt;
         decode(w, tt, nt);
         const int y0 = tt * kTok + rank * 128, y1 = nt * kFeat + rank * 128;
-        int kx = (nt * 13) % ktiles;   // PAIR_ROT
+        // Rows of long k lie far apart, and a k tile at a time is 128 bytes from each: there the group's first pair brings the weights of eight k
+        // tiles at a time to L2 (17408 k, 5120 features: 512 tokens 155 -> 130 us, 4096 685 -> 544; at 5120 k it costs 8 %, and at 8192
+        // tokens the other operand sets the pace).
+        const bool lead = p.K >= 8192 && tt_all <= 2 * kGroup && tt % kGroup == 0;
         for (int kt = 0; kt < ktiles; ++kt) {
+          if (lead && kt % 8 == 0) {
+            const int k1 = min(kt + 16, ktiles);
+            for (int k = kt == 0 ? 0 : kt + 8; k < k1; ++k) tma_prefetch_2d(&tmW, k * 64, y1);
+          }
           ok = mbar_wait(&empty[st.idx], st.phase ^ 1, abort_flag);
           if (!ok) break;
           if (rank == 0) mbar_expect_tx(&full[st.idx], 2 * kStage);   // the other CTA's bytes too; they may land before this
           const uint32_t bar = mapa_shared(smem_u32(&full[st.idx]), 0);
           uint8_t* dst = smem + st.idx * kStage;
-          tma_load_2d_pair(dst, &tmX, kx * 64, y0, bar);              // rows past the tensors are zero-filled
-          tma_load_2d_pair(dst + kHalfBytes, &tmW, kx * 64, y1, bar);
-          if (++kx == ktiles) kx = 0;
+          tma_load_2d_pair(dst, &tmX, kt * 64, y0, bar);              // rows past the tensors are zero-filled
+          tma_load_2d_pair(dst + kHalfBytes, &tmW, kt * 64, y1, bar);
           st.advance(kStages);
         }
       }

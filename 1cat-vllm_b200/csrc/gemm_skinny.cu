@@ -101,23 +101,20 @@ __global__ void __launch_bounds__(32 * kMaxWarps) gemm_skinny_kernel(const GemmP
 
   // copies: lane -> row `lane` of the warp's 32 for the four quarters of a unit (eight lanes copy 128 neighbouring bytes). Everything a copy needs
   // is a lane's constant plus a pointer that moves on by a constant.
-  // ROT_COMMENT
-  const int rot = (int)((blockIdx.x * 13u) % (unsigned)units);
-  auto unit_at = [&](int v) { return v + rot < units ? v + rot : v + rot - units; };
-  const uint8_t* wsrc = p.w4 + (size_t)nt * ktiles * Q::kTileBytes + (rt + lane) * 16;
+  const uint8_t* wsrc = p.w4 + ((size_t)nt * ktiles + wk * Q::kTiles) * Q::kTileBytes + (rt + lane) * 16;
+  const size_t wstep = (size_t)WK * Q::kTiles * Q::kTileBytes;
   const uint32_t* zsrc = p.w4_sz + ((size_t)nt * 128 + rt + lane) * Q::kScaleWords;
   uint32_t wdst[4];                      // quarter q of a row lies at q ^ (row / 2 % 4): neighbouring rows in different banks
 #pragma unroll
   for (int q = 0; q < 4; ++q) wdst[q] = lane * 64 + ((q ^ ((lane >> 1) & 3)) << 4);
   const uint32_t zdst = kUnitBytes + lane * (4 * Q::kScaleWords);
-  auto copy_weights = [&](int v, uint32_t dst) {
-    const int u = unit_at(v);
-    const uint8_t* src = wsrc + (size_t)u * (Q::kTiles * Q::kTileBytes);
+  auto copy_weights = [&](int u, uint32_t dst) {
     // 4-bit: quarters 0, 1 are the halves of the first tile, 2, 3 of the second (missing when the number of tiles is odd: its activations are 0)
     const bool whole = Q::kFp8 || u * 2 + 1 < ktiles;
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-      if (q < 2 || whole) cp16(dst + wdst[q], src + q * 2048);
+      if (q < 2 || whole) cp16(dst + wdst[q], wsrc + q * 2048);
+    wsrc += wstep;
 #pragma unroll
     for (int i = 0; i < Q::kTiles; ++i) {
       const int kt = u * Q::kTiles + (whole ? i : 0);
@@ -132,13 +129,12 @@ __global__ void __launch_bounds__(32 * kMaxWarps) gemm_skinny_kernel(const GemmP
   // chunk c lies at c ^ (c / 4) ^ (row % 2) (4-bit) or c ^ (row % 2) (fp8): the four quarters of two rows in different banks
   const int xc = lane % XCH, xr = lane / XCH;
   const uint32_t xdst = kUnitBytes + Q::kScaleBytes + xr * Q::kXRow + ((Q::kFp8 ? xc ^ (xr & 1) : xc ^ (xc >> 2) ^ (xr & 1)) << 4);
-  const __nv_bfloat16* xsrc = x + (size_t)xr * ldx + xc * 8;
-  const size_t xrows = (size_t)XR * ldx;
+  const __nv_bfloat16* xsrc = x + (size_t)xr * ldx + wk * Q::kK + xc * 8;
+  const size_t xstep = (size_t)WK * Q::kK, xrows = (size_t)XR * ldx;
   const int k_left = p.K - xc * 8;
-  auto copy_x = [&](int v, uint32_t dst) {
-    const int u = unit_at(v);
+  auto copy_x = [&](int u, uint32_t dst) {
     const bool there = u * Q::kK < k_left;
-    const __nv_bfloat16* src = xsrc + (size_t)u * Q::kK;
+    const __nv_bfloat16* src = xsrc;
     int left = nvalid - xr;
 #pragma unroll
     for (int r = 0; r < NB * 8; r += XR) {
@@ -146,6 +142,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps) gemm_skinny_kernel(const GemmP
       left -= XR;
       src += xrows;
     }
+    xsrc += xstep;
   };
 #pragma unroll
   for (int i = 0; i < kStages - 1; ++i)

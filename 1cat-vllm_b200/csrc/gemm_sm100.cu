@@ -239,8 +239,7 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     k1 = min(k0 + p.ktiles_per_split, ktiles);
   };
   const bool grouped = p.work != nullptr;
-  // ROT_COMMENT
-  auto rotation = [&](int nt, int len) { return WKIND >= 1 ? (nt * 13) % len : 0; };
+
 
   // ------------------------------------------------------------------ epilogue (run by the epilogue warps, or by the first
   // dequantisation group of a SMALL CTA)
@@ -494,7 +493,6 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x) {
         int nt, tt, sp_, k0, k1;
         decode(w, nt, tt, sp_, k0, k1);
-        int kx = k0 + rotation(nt, k1 - k0);   // the k tile that is copied next
         for (int kt = k0; kt < k1; kt += KPS) {
           const int kc = min(KPS, k1 - kt);
           ok = mbar_wait(&empty[st.idx], st.phase ^ 1, abort_flag);
@@ -502,9 +500,8 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
           mbar_expect_tx(&full[st.idx], bytes * kc);
           for (int j = 0; j < kc; ++j) {
             for (int i = 0; i < NT; ++i)  // rows past T are zero-filled by the copy
-              tma_load_2d(sx + ((st.idx * KPS + j) * NT + i) * xs, &tmX, kx * BK, grouped ? tt : (tt * NT + i) * tn, &full[st.idx]);
-            if (WKIND == 0) tma_load_2d(sw + (st.idx * KPS + j) * kWStageBytes, &tmW, kx * BK, nt * BM, &full[st.idx]);
-            if (++kx == k1) kx = k0;
+              tma_load_2d(sx + ((st.idx * KPS + j) * NT + i) * xs, &tmX, (kt + j) * BK, grouped ? tt : (tt * NT + i) * tn, &full[st.idx]);
+            if (WKIND == 0) tma_load_2d(sw + (st.idx * KPS + j) * kWStageBytes, &tmW, (kt + j) * BK, nt * BM, &full[st.idx]);
           }
           st.advance(S);
         }
@@ -519,10 +516,9 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x) {
         int nt, tt, sp_, k0, k1;
         decode(w, nt, tt, sp_, k0, k1);
-        int kx = k0 + rotation(nt, k1 - k0);
-        const uint8_t* wsrc = p.w4 + ((size_t)nt * ktiles + kx) * kPackedBytes;
+        const uint8_t* wsrc = p.w4 + ((size_t)nt * ktiles + k0) * kPackedBytes;
         const uint32_t* zsrc = p.w4_sz + (size_t)nt * BM * sz_words(WKIND);
-        int g = kx / gk, gi = kx - g * gk;  // quantisation group of the k tile and position inside it
+        int g = k0 / gk, gi = k0 - g * gk;  // quantisation group of the k tile and position inside it
         for (int kt = k0; kt < k1; ++kt) {
           ok = mbar_wait(&pempty[pr.idx], pr.phase ^ 1, abort_flag);
           if (!ok) break;
@@ -533,12 +529,6 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
           bulk_load(dst + kPackedBytes, zsrc + (size_t)g * p.n_pad * sz_words(WKIND), sz_bytes(WKIND), &pfull[pr.idx]);
           wsrc += kPackedBytes;
           if (++gi == gk) { gi = 0; ++g; }
-          if (++kx == k1) {                 // round to the beginning of the range
-            kx = k0;
-            wsrc = p.w4 + ((size_t)nt * ktiles + k0) * kPackedBytes;
-            g = k0 / gk;
-            gi = k0 - g * gk;
-          }
           pr.advance(PS);
         }
       }

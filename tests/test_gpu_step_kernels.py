@@ -333,3 +333,24 @@ def test_gated_norm_in_wide_accesses(T, heads, D):
     z = wide[:, heads * D:]
     y = K().rms_norm_gated(x.cuda(), wide.cuda()[:, heads * D:], w.cuda(), 1e-6, heads)
     _close(y.view(T, heads, D), ref.rms_norm_gated(x.view(T, heads, D), z.reshape(T, heads, D), w, 1e-6), 2 ** -6, 2 ** -8)
+
+
+@pytest.mark.parametrize("kind,T,N,Kd,splits", [(1, 4, 1792, 1024, 0), (2, 12, 1792, 1024, 0), (1, 32, 1024, 1152, 1), (2, 200, 1024, 1024, 1), (0, 600, 20480, 1152, 0)])
+def test_a_weight_row_sums_alike_in_a_layer_and_in_a_slice_of_it(kind, T, N, Kd, splits):
+    """The order of a sum over k depends on no feature tile's number: the second half of the rows, as a layer of its own (a rank's slice), gives the same bits."""
+    g = torch.Generator().manual_seed(N)
+    x = torch.randn(T, Kd, generator=g).bfloat16().cuda()
+    if kind == 0:
+        w = (torch.randn(N, Kd, generator=g) * Kd ** -0.5).bfloat16().cuda()
+        whole, half = (K().gemm_bf16(x, t, out_dtype=torch.float32) for t in (w, w[N // 2:]))
+    else:
+        c = torch.randint(0, 16, (N, Kd), generator=g, dtype=torch.uint8) if kind == 1 else torch.randn(N, Kd, generator=g).to(torch.float8_e4m3fn).view(torch.uint8)
+        z, s = torch.randint(0, 16, (N, Kd // 128), generator=g, dtype=torch.uint8), torch.rand(N, Kd // 128, generator=g) * 0.02 + 0.001
+
+        def product(lo):
+            t = [v[lo:].contiguous().cuda() for v in (c, z, s)]
+            tiles, sz, npad = K().pack_w4(*t, 128)[:3] if kind == 1 else K().pack_fp8(t[0], t[2], 128)[:3]
+            out = torch.empty(T, N - lo, dtype=torch.bfloat16, device="cuda")
+            return K()._gemm(x, None, tiles, sz, out, None, N - lo, N - lo, N - lo, npad, 0, 2, force_splits=splits, wkind=kind)
+        whole, half = product(0), product(N // 2)
+    assert torch.equal(whole[:, N // 2:], half)
