@@ -30,6 +30,8 @@ void gemm(torch::Tensor x, c10::optional<torch::Tensor> w, c10::optional<torch::
           torch::Tensor out, c10::optional<torch::Tensor> bias, torch::Tensor ws, torch::Tensor counters, int64_t N, int64_t n_rows,
           int64_t n_out, int64_t n_pad, int64_t epi, int64_t group_ktiles, int64_t force_splits, int64_t force_tn,
           std::vector<int64_t> push_dst, int64_t push_rows, int64_t wkind, int64_t trace_ptr, int64_t push_sel, int64_t push_sel_stride) {
+  // only bf16 weights have fp32 results and GELU epilogues: the kernels of packed ones have no other store
+  TORCH_CHECK(w.has_value() != w4.has_value(), "exactly one form of the weight is given");
   check_bf16(x, "x");
   const bool f32_out = out.scalar_type() == torch::kFloat32;
   if (f32_out) {

@@ -385,7 +385,8 @@ int gemm_widen_rows(const GemmParams& p, int num_sms) { return plan_slabs(p, num
 // these estimates say that it wins by 5 %. Measured (us), int4: 34816 x 5120 at 8192 tokens 1939 for 2730, at 1087 tokens 520 for 383 in small
 // slabs; 5120 x 17408 at 1087 tokens 400 for 187.
 bool gemm_widen_takes(const GemmParams& p, int num_sms) {
-  if (p.w4 == nullptr || p.wkind < 1 || p.wkind > 4 || p.T < kWidenTokens || !gemm_pair_takes(p, num_sms)) return false;
+  if (p.w4 == nullptr || p.wkind < 1 || p.wkind > 4 || p.out == nullptr || p.out_f32 != nullptr || (p.epi != EPI_STORE && p.epi != EPI_SILU_MUL)) return false;
+  if (p.T < kWidenTokens || !gemm_pair_takes(p, num_sms)) return false;
   const long long n = (p.n_rows + 127) / 128, w1 = (n * ((p.T + 191) / 192) + num_sms - 1) / num_sms, w2 = (n * ((p.T + 383) / 384) + num_sms - 1) / num_sms;
   const double one = w1 * 0.45, two = w2 * 0.72, tile_by_tile = (p.K / 64) * (one < two ? one : two) + 20.0;
   return plan_slabs(p, num_sms).us < 0.95 * tile_by_tile;

@@ -354,3 +354,14 @@ def test_a_weight_row_sums_alike_in_a_layer_and_in_a_slice_of_it(kind, T, N, Kd,
             return K()._gemm(x, None, tiles, sz, out, None, N - lo, N - lo, N - lo, npad, 0, 2, force_splits=splits, wkind=kind)
         whole, half = product(0), product(N // 2)
     assert torch.equal(whole[:, N // 2:], half)
+
+
+@pytest.mark.parametrize("T,dtype,epi", [(40, torch.float32, 0), (1100, torch.float32, 0), (40, torch.bfloat16, 2), (1100, torch.bfloat16, 3)])
+def test_packed_gemm_refuses_a_second_form_of_its_weight(T, dtype, epi):
+    """fp32 results and GELU epilogues are those of bf16 weights; a bf16 weight beside the packed one does not open them."""
+    N, Kd = 5120, 192
+    tiles, sz, npad = K().pack_fp8(torch.zeros(N, Kd, dtype=torch.uint8, device="cuda"), torch.ones(N, Kd // 64, device="cuda"), 64)
+    x, w = torch.zeros(T, Kd, device="cuda").bfloat16(), torch.zeros(N, Kd, device="cuda").bfloat16()
+    n = N // 2 if epi == 3 else N
+    with pytest.raises(RuntimeError, match="one form of the weight"):
+        K()._gemm(x, w, tiles, sz, torch.empty(T, n, dtype=dtype, device="cuda"), None, N, N, n, npad, epi, 1, wkind=2)
