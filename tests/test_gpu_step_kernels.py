@@ -14,7 +14,7 @@ def K():
 
 def _close(a, b, rtol, atol, what=""):
     a, b = a.float().cpu(), b.float().cpu()
-    bad = (a - b).abs() > atol + rtol * b.abs()
+    bad = ~((a - b).abs() <= atol + rtol * b.abs())   # NaN is a difference
     assert not bad.any(), f"{what}: {int(bad.sum())} of {bad.numel()} differ, largest by {float((a - b).abs().max())}"
 
 
