@@ -379,9 +379,9 @@ int make_tmap(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t cols, u
 
 // Prefill attention of every request with more than `short_q_len` query tokens. `num_q_tiles` = sum over those requests of
 // ceil(q_len / 256); `num_blocks` = pages in the cache. Needs D == 128, the heads of a token contiguous in q (q_sh == D),
-// 16-byte aligned bases and pitches.
+// 16-byte aligned bases and pitches, and a positive scale (maxima are taken and keys masked ahead of it).
 int attention_prefill_tc_launch(const AttnParams& p, long long num_blocks, cudaStream_t st) {
-  if (p.D != HD || p.q_sh != HD || p.Hq % p.Hkv || p.bs < 16 || (p.bs & (p.bs - 1))) return -1;
+  if (p.D != HD || p.q_sh != HD || !(p.scale > 0.f) || p.Hq % p.Hkv || p.bs < 16 || (p.bs & (p.bs - 1))) return -1;
   if (((uintptr_t)p.q & 15) || ((uintptr_t)p.kv_cache & 15) || ((uintptr_t)p.out & 15) || (p.q_st * 2) % 16) return -1;
   if (p.num_q_tiles <= 0) return 0;
   if (p.num_q_tiles > 65535) return -1;

@@ -584,7 +584,7 @@ def paged_attention(q, kv_cache, md, scale, out=None, lse=None, window=0, softca
                            md.max_query_len, short, ws_o, ws_ml, window, softcap, sinks, 1.0, 1.0, keep, bias_table, gate, chunk)
         _LAUNCHES += 2 if splits > 1 else 1
     if tiles:
-        if (D == 128 and q.stride(1) == D and _ATTN_PREFILL_TC and not window and not softcap and sinks is None and not extended
+        if (D == 128 and q.stride(1) == D and _ATTN_PREFILL_TC and scale > 0 and not window and not softcap and sinks is None and not extended
                 and kv_cache.dtype == torch.bfloat16):
             # tcgen05 kernel: 256 query tokens per CTA
             tiles_tc = sum(-(-x // 256) for x in md.query_lens_cpu if x > short)

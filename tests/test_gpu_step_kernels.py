@@ -252,6 +252,20 @@ def test_prompt_attention_in_pairs_of_query_tiles(qlens, ctxs, Hq, Hkv, scale):
     _close(lse[qsl[1] - 1, : Hq // Hkv], torch.logsumexp(s, -1), 1e-3, 1e-2, "lse")
 
 
+@pytest.mark.parametrize("scale", [0.0, -0.1])
+def test_prompt_attention_with_a_scale_of_zero_or_less(scale):
+    """The tcgen05 kernel takes a row's maximum and masks keys ahead of the scale: such a scale stays with the kernel that scales first."""
+    from onecat_vllm.worker.attn_metadata import AttentionMetadata
+    Hq, Hkv, D, n = 4, 2, 128, 300
+    g = torch.Generator().manual_seed(1)
+    cache, q = torch.randn(20, 2, Hkv, 16, D, generator=g).bfloat16(), torch.randn(n, Hq, D, generator=g).bfloat16()
+    bt, qsl, sl = torch.arange(1, 20, dtype=torch.int32).view(1, -1), torch.tensor([0, n], dtype=torch.int32), torch.tensor([n], dtype=torch.int32)
+    md = AttentionMetadata(1, n, qsl.cuda(), sl.cuda(), bt.cuda(), None, None, n, n, query_lens_cpu=[n], seq_lens_cpu=[n])
+    out = K().paged_attention(q.cuda(), cache.cuda(), md, scale)
+    assert K().check_status() == 0
+    _close(out, ref.paged_attention(q, cache, bt, qsl, sl, scale), 2e-2, 1e-2)
+
+
 @pytest.mark.parametrize("T,N,Kd,epi,bias,f32", [(256, 9472, 64, 0, False, False), (300, 5120, 640, 0, True, False), (2500, 1000, 1088, 0, True, True), (129, 9600, 128, 1, False, False),
                                                  (1030, 2112, 448, 3, False, False), (515, 3336, 192, 2, True, False), (9000, 520, 256, 0, False, False)])
 def test_gemm_over_pairs_of_sms(T, N, Kd, epi, bias, f32):
