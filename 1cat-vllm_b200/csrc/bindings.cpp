@@ -1277,13 +1277,14 @@ torch::Tensor sigmoid_mul(torch::Tensor x, torch::Tensor gate) {
   return y;
 }
 
-// Addresses of the translation units' status words on the current device.
-static const oc::StatusWords& status_words() {
+// Addresses of the translation units' status words on the current device; null when the runtime has none to give (no device, or one that
+// has failed).
+static const oc::StatusWords* status_words() {
   static std::mutex m;
   static oc::StatusWords words[64] = {};
   std::lock_guard<std::mutex> lock(m);
-  const int dev = c10::cuda::current_device();
-  TORCH_CHECK(dev >= 0 && dev < 64, "device index");
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
   oc::StatusWords& w = words[dev];
   if (w.n == 0) {
     oc::StatusWords t{};
@@ -1292,22 +1293,27 @@ static const oc::StatusWords& status_words() {
                      oc::mla_prefill_status_word, oc::diff_prefill_status_word, oc::talk_prefill_status_word, oc::mla_decode_tc_status_word,
                      oc::gemm_pair_status_word}) {
       unsigned int* p = get();
-      TORCH_CHECK(p != nullptr, "a status word has no address");
+      if (p == nullptr) return nullptr;
       t.w[t.n++] = p;
     }
     w = t;
   }
-  return w;
+  return &w;
 }
 
 // Enqueues one kernel that writes every status word into `pinned` (int32, >= 16 entries, pinned host memory) on the current stream; the
 // caller reads them after an event recorded behind this call (async scheduling: no device-wide synchronisation).
 void read_status_async(torch::Tensor pinned) {
   TORCH_CHECK(pinned.scalar_type() == torch::kInt32 && pinned.numel() >= 16 && !pinned.is_cuda() && pinned.is_pinned(), "need 16 pinned int32 words");
-  TORCH_CHECK(oc::status_gather_launch(status_words(), reinterpret_cast<unsigned int*>(pinned.data_ptr<int>()), cur_stream()) == 0, "status gather failed");
+  const oc::StatusWords* w = status_words();
+  TORCH_CHECK(w != nullptr && oc::status_gather_launch(*w, reinterpret_cast<unsigned int*>(pinned.data_ptr<int>()), cur_stream()) == 0, "status gather failed");
 }
 
-int64_t read_status(bool clear) { return (int64_t)oc::status_read(status_words(), clear); }
+// 0x80000000: the device cannot be asked.
+int64_t read_status(bool clear) {
+  const oc::StatusWords* w = status_words();
+  return w != nullptr ? (int64_t)oc::status_read(*w, clear) : (int64_t)0x80000000u;
+}
 
 // ---- symmetric slab + peer-memory reductions
 int64_t comm_alloc(int64_t bytes) {
