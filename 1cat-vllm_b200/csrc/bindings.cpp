@@ -935,7 +935,10 @@ torch::Tensor mla_decode(torch::Tensor q_abs, torch::Tensor q_rope, torch::Tenso
   return out;
 }
 
-bool mla_decode_wide(int64_t kv_lora) { return oc::mla_decode_tc_takes((int)kv_lora, 64, 16, 0, 1.f); }
+// whether calls of this form run the tcgen05 kernel (their splits are planned for it)
+bool mla_decode_wide(int64_t kv_lora, int64_t rope_pad, int64_t page, bool fine, double scale) {
+  return oc::mla_tensor_core_sizes((int)kv_lora, (int)rope_pad) && oc::mla_decode_tc_takes((int)kv_lora, (int)rope_pad, (int)page, fine ? 1 : 0, (float)scale);
+}
 bool mla_tensor_core_sizes(int64_t kv_lora, int64_t rope_pad) { return oc::mla_tensor_core_sizes((int)kv_lora, (int)rope_pad); }
 
 // Expanded-form prefill, first half: the contexts of the listed requests gathered from their pages and the query rows in whole chunks.

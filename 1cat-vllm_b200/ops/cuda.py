@@ -819,11 +819,16 @@ def per_head_matmul(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     return out
 
 
-def plan_mla_splits(H: int, lora: int, query_lens: list, seq_lens: list, num_sms: int) -> int:
-    """KV splits of a latent-attention launch: as many CTAs fit an SM as two key tiles and the queries leave room for. The tcgen05 kernel has
-    one CTA per SM and two of them (halves of the output columns) per 128 rows, which need about
+def mla_decode_wide(lora: int, rope_pad: int, page: int, fine: bool, scale: float) -> bool:
+    """Whether bf16 latent attention of this form runs the tcgen05 kernel: 128 rows a CTA, where the mma.sync one takes 16."""
+    return _C.mla_decode_wide(lora, rope_pad, page, fine, scale)
+
+
+def plan_mla_splits(H: int, lora: int, query_lens: list, seq_lens: list, num_sms: int, wide: bool) -> int:
+    """KV splits of a latent-attention launch: as many CTAs fit an SM as two key tiles and the queries leave room for. The tcgen05 kernel
+    (``wide``: see ``mla_decode_wide``) has one CTA per SM and two of them (halves of the output columns) per 128 rows, which need about
     6 us to start and 1.3 us per key tile (measured: 97 us at 32 requests x 4096 keys x 128 heads in two splits)."""
-    if _C.mla_decode_wide(lora):
+    if wide:
         return choose_decode_splits(2 * sum(-(-q * H // 128) for q in query_lens), max(seq_lens), num_sms, 1, start=6.0, tile=1.3)
     per_sm = max(1, min(4, (227 << 10) // ((16 + 2 * 64) * (lora + 64) * 2 + 6144)))
     return choose_decode_splits(len(query_lens) * -(-max(query_lens) * H // 16), max(seq_lens), num_sms, per_sm)
@@ -848,7 +853,8 @@ def mla_decode(q_abs, q_pe, latent_cache, md, scale, lora, cos_sin=None, interle
         if static and plan is not None and plan[0][0] == "mla":
             splits = plan[1][2]  # captured decode graph: the split count is part of the graph's key
         else:
-            splits = plan_mla_splits(H, lora, ql, sl, _sms(q_abs.device))
+            wide = mla_decode_wide(lora, latent_cache.shape[-1] - lora, latent_cache.shape[1], fine, scale)
+            splits = plan_mla_splits(H, lora, ql, sl, _sms(q_abs.device), wide)
         if splits > 1:
             w = workspace(q_abs.device)
             ws_o, ws_ml = (w.attn_static if static else w.attn)(splits * T * H * lora, splits * T * H * 4)   # a reference and a sum for each half of the columns

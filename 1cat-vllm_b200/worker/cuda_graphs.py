@@ -44,7 +44,10 @@ class DecodeGraphs:
         self.own_plans = any(getattr(a, "chunk", 0) or getattr(a, "diff", None) is not None or a.kv_shared or a.window_keep or a.bias_table is not None or (a.Hq, a.Hkv, a.D) != (attns[0].Hq, attns[0].Hkv, attns[0].D)
                              for a in attns)
         mlas = [l.self_attn for l in mla]
-        self.own_plans = self.own_plans or bool(mla) and (bool(layers) or any((a.H, a.lora_pad) != (mlas[0].H, mlas[0].lora_pad) for a in mlas)) or not (layers or mla)
+        # latent attention: the splits are those of the kernel that its calls run
+        forms = {(a.H, a.lora_pad, K.mla_decode_wide(a.lora_pad, a.rope_pad, runner.block_size, a.fine_weights, a.scale)) for a in mlas}
+        self.own_plans = self.own_plans or bool(mla) and (bool(layers) or len(forms) > 1) or not (layers or mla)
+        self.mla_wide = all(wide for *_, wide in forms)
         self.max_span = 0   # the longest stretch of keys that a decode row of any layer walks (0: the whole context)
         if layers:
             a = layers[0].self_attn
@@ -80,7 +83,7 @@ class DecodeGraphs:
             return rp, q, self._context_bucket(max_seq)
         from onecat_vllm.ops.cuda import _sms, choose_decode_splits, plan_mla_splits
         if self.geom[0] == "mla":
-            want = plan_mla_splits(self.geom[1], self.geom[2], [q] * rp, [max_seq], _sms(self.r.device))
+            want = plan_mla_splits(self.geom[1], self.geom[2], [q] * rp, [max_seq], _sms(self.r.device), self.mla_wide)
         else:
             want = choose_decode_splits(rp * self.geom[1], max_seq, _sms(self.r.device))
         s = 1  # bucketed to powers of two (rounding up keeps the grid sized for the live context)

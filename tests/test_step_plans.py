@@ -8,3 +8,21 @@ def test_status_of_a_device_that_cannot_be_asked():
     """The worst status instead of an exception: failure detection reads a number."""
     from onecat_vllm.ops import _C
     assert _C.read_status(False) == 0x80000000 and _C.read_status(True) == 0x80000000
+
+
+@pytest.mark.parametrize("form,wide", [(dict(), True), (dict(fine=True), False), (dict(page=8), False), (dict(rope_pad=128), False), (dict(lora=256), False), (dict(scale=-1.0), False)])
+def test_latent_attention_is_split_for_the_kernel_that_runs(form, wide, monkeypatch):
+    """The tcgen05 kernel's plan (one CTA an SM, 128 rows each) only for calls that it takes: the others keep the splits of 16-row tiles, in eager
+    calls and in captured graphs."""
+    from types import SimpleNamespace
+    from onecat_vllm.ops import cuda as K
+    from onecat_vllm.worker.cuda_graphs import DecodeGraphs
+    f = dict(dict(lora=512, rope_pad=64, page=16, fine=False, scale=0.07), **form)
+    assert K.mla_decode_wide(**f) == wide
+    H, R, ctx = 16, 32, 4096
+    per_sm = max(1, min(4, (227 << 10) // ((16 + 2 * 64) * (f["lora"] + 64) * 2 + 6144)))
+    want = K.choose_decode_splits(2 * R, ctx, 148, 1, start=6.0, tile=1.3) if wide else K.choose_decode_splits(R, ctx, 148, per_sm)
+    assert K.plan_mla_splits(H, f["lora"], [1] * R, [ctx], 148, K.mla_decode_wide(**f)) == want
+    monkeypatch.setattr(K, "_sms", lambda device: 148)
+    graphs = SimpleNamespace(eligible=True, sizes=[R], max_q=1, own_plans=False, geom=("mla", H, f["lora"]), mla_wide=wide, r=SimpleNamespace(device=None))
+    assert DecodeGraphs.plan(graphs, R, 1, ctx) == (R, 1, 1 << (want - 1).bit_length())
