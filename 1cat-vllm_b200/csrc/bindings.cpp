@@ -894,7 +894,7 @@ static void check_sink_gate(const c10::optional<torch::Tensor>& sinks, const c10
 torch::Tensor mla_decode(torch::Tensor q_abs, torch::Tensor q_rope, torch::Tensor cache, torch::Tensor qsl, torch::Tensor seq_lens,
                          torch::Tensor block_table, double scale, int64_t max_q_len, int64_t splits, c10::optional<torch::Tensor> ws_o,
                          c10::optional<torch::Tensor> ws_ml, c10::optional<torch::Tensor> cos_sin, bool interleaved, bool fine, int64_t skip_min_len,
-                         c10::optional<torch::Tensor> sinks, c10::optional<torch::Tensor> gate) {
+                         c10::optional<torch::Tensor> sinks, c10::optional<torch::Tensor> gate, bool wide) {
   const auto et = q_abs.scalar_type();
   TORCH_CHECK(q_abs.is_cuda() && (et == torch::kBFloat16 || et == torch::kFloat32) && q_rope.scalar_type() == et && cache.scalar_type() == et, "bf16 or fp32 throughout");
   TORCH_CHECK(q_abs.is_contiguous() && cache.is_contiguous() && cache.dim() == 3 && q_rope.dim() == 3 && q_rope.stride(2) == 1, "q and cache layouts");
@@ -919,6 +919,7 @@ torch::Tensor mla_decode(torch::Tensor q_abs, torch::Tensor q_rope, torch::Tenso
   p.bt_stride = (int)block_table.stride(0); p.R = (int)seq_lens.size(0);
   p.bs = (int)cache.size(1); p.bs_shift = 0;
   p.num_blocks = (int)cache.size(0);
+  p.wide = wide ? 1 : 0;
   p.halves = 1;
   while ((1 << p.bs_shift) < p.bs) ++p.bs_shift;
   p.max_q_len = (int)max_q_len; p.splits = (int)splits; p.scale = (float)scale;

@@ -242,6 +242,7 @@ struct MlaParams {
   const void* gate;             // [T][H] (row pitch gate_st): outputs are multiplied by its sigmoid, or null
   long long gate_st;
   int num_blocks;               // pages of the cache
+  int wide;                     // the tcgen05 kernel (128 rows a CTA) instead of the mma.sync one (16)
   int halves;                   // 2: ws_ml holds the reference and sum of each half of the columns, else 1
 };
 bool mla_decode_tc_takes(int kv_lora, int rope_pad, int bs, int fine, float scale);

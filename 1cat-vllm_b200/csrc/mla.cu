@@ -479,7 +479,8 @@ int mla_decode_launch(const MlaParams& p, cudaStream_t st) {
   if (p.bs < 1 || (p.bs & (p.bs - 1)) || p.splits < 1 || p.splits > 32) return -1;
   if (p.f32) return p.splits == 1 ? plain_e<float>(p, st) : -1;
   if (!mla_tensor_core_sizes(p.kv_lora, p.rope_pad)) return p.splits == 1 ? plain_e<__nv_bfloat16>(p, st) : -1;
-  if (mla_decode_tc_takes(p.kv_lora, p.rope_pad, p.bs, p.fine, p.scale)) {
+  if (p.wide) {
+    if (!mla_decode_tc_takes(p.kv_lora, p.rope_pad, p.bs, p.fine, p.scale)) return -1;
     MlaParams w = p;
     w.halves = 2;
     const int rc = mla_decode_tc_launch(w, st);

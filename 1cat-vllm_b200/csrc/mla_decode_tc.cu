@@ -426,10 +426,10 @@ int make_tmap(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t cols, u
 
 }  // namespace
 
-// Which launches take this kernel: DeepSeek's latent width, weights in one term, pages of whole 16-key pieces (a TMA box) and positive scales
-// (the maximum is taken before scaling). With 16 heads seven eighths of a tile's rows are padding and it is still the faster one (32 requests
-// x 4096 keys: 89 us against 122; one request x 1000 keys: 30 against 46): the tensor core reads a key tile once where mma.sync kept
-// four warps busy with fragments.
+// What this kernel can run: DeepSeek's latent width, weights in one term, pages of whole 16-key pieces (a TMA box) and positive scales
+// (the maximum is taken before scaling). Callers choose (plan_mla in ops/cuda.py): with 16 rows of heads a request seven eighths of a tile are
+// padding and it is mostly still the faster one (32 requests x 4096 keys: 89 us against 122; one request x 1000 keys: 30 against 46), since the
+// tensor core reads a key tile once where mma.sync kept four warps busy with fragments.
 bool mla_decode_tc_takes(int kv_lora, int rope_pad, int bs, int fine, float scale) {
   return kv_lora == DV && rope_pad <= 64 && rope_pad % 8 == 0 && !fine && scale > 0.f && bs >= 16 && (bs & (bs - 1)) == 0;
 }

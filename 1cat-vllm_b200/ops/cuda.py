@@ -824,14 +824,23 @@ def mla_decode_wide(lora: int, rope_pad: int, page: int, fine: bool, scale: floa
     return _C.mla_decode_wide(lora, rope_pad, page, fine, scale)
 
 
-def plan_mla_splits(H: int, lora: int, query_lens: list, seq_lens: list, num_sms: int, wide: bool) -> int:
-    """KV splits of a latent-attention launch: as many CTAs fit an SM as two key tiles and the queries leave room for. The tcgen05 kernel
-    (``wide``: see ``mla_decode_wide``) has one CTA per SM and two of them (halves of the output columns) per 128 rows, which need about
-    6 us to start and 1.3 us per key tile (measured: 97 us at 32 requests x 4096 keys x 128 heads in two splits)."""
-    if wide:
-        return choose_decode_splits(2 * sum(-(-q * H // 128) for q in query_lens), max(seq_lens), num_sms, 1, start=6.0, tile=1.3)
+def plan_mla(H: int, lora: int, query_lens: list, seq_lens: list, num_sms: int, wide: bool) -> tuple[int, bool]:
+    """(KV splits, whether the tcgen05 kernel runs) of a latent-attention launch; ``wide``: it can (see ``mla_decode_wide``). As many CTAs of
+    the mma.sync kernel fit an SM as two key tiles and the queries leave room for. The tcgen05 kernel has one CTA per SM and two of them (halves of
+    the output columns) per 128 rows, which need about 6 us to start and 1.3 us per key tile (measured: 97 us at 32 requests x 4096 keys x 128
+    heads in two splits).
+
+    Requests of at most 16 rows are one CTA of the mma.sync kernel, and two of the other however few their rows. Where that is more waves
+    of CTAs and contexts are short, the former is faster: a wave takes 0.6 + 0.65 us per row + 6.2 us per key tile there, 9.8 + 2.1 us per
+    key tile here. Measured (us, mma.sync / tcgen05), 16 heads: 128 requests x 64 keys 24.6 / 30.7, x 190 34.8 / 36.9, x 256 41 / 41, x 400
+    59 / 55; 256 x 64 42 / 53; 149 x 64 37 / 41, x 100 49 / 45; 74 x 16 23.8 / 18.4."""
+    n, rows, tiles = len(query_lens), max(query_lens) * H, -(-max(seq_lens) // 64)
+    waves, waves_wide = -(-n // num_sms), -(-2 * n // num_sms)
+    few = rows <= 16 and waves < waves_wide and waves * (0.6 + 0.65 * rows + 6.2 * tiles) < waves_wide * (9.8 + 2.1 * tiles)
+    if wide and not few:
+        return choose_decode_splits(2 * sum(-(-q * H // 128) for q in query_lens), max(seq_lens), num_sms, 1, start=6.0, tile=1.3), True
     per_sm = max(1, min(4, (227 << 10) // ((16 + 2 * 64) * (lora + 64) * 2 + 6144)))
-    return choose_decode_splits(len(query_lens) * -(-max(query_lens) * H // 16), max(seq_lens), num_sms, per_sm)
+    return choose_decode_splits(n * -(-rows // 16), max(seq_lens), num_sms, per_sm), False
 
 
 def mla_decode(q_abs, q_pe, latent_cache, md, scale, lora, cos_sin=None, interleaved=True, fine=False, skip_min_len=0, sinks=None, gate=None):
@@ -842,7 +851,7 @@ def mla_decode(q_abs, q_pe, latent_cache, md, scale, lora, cos_sin=None, interle
     global _LAUNCHES
     T, H, _ = q_abs.shape
     ws_o = ws_ml = None
-    splits = 1
+    splits, wide = 1, False
     ql, sl = md.query_lens_cpu or [md.max_query_len] * md.num_reqs, md.seq_lens_cpu or [md.max_seq_len]
     if skip_min_len:
         keep = [(q, s) for q, s in zip(ql, sl) if 0 < q < skip_min_len]
@@ -851,16 +860,16 @@ def mla_decode(q_abs, q_pe, latent_cache, md, scale, lora, cos_sin=None, interle
         static = getattr(md, "static_ws", False)
         plan = getattr(md, "attn_plan", None)
         if static and plan is not None and plan[0][0] == "mla":
-            splits = plan[1][2]  # captured decode graph: the split count is part of the graph's key
+            splits, wide = plan[1][2]  # captured decode graph: both are part of the graph's key
         else:
             wide = mla_decode_wide(lora, latent_cache.shape[-1] - lora, latent_cache.shape[1], fine, scale)
-            splits = plan_mla_splits(H, lora, ql, sl, _sms(q_abs.device), wide)
+            splits, wide = plan_mla(H, lora, ql, sl, _sms(q_abs.device), wide)
         if splits > 1:
             w = workspace(q_abs.device)
             ws_o, ws_ml = (w.attn_static if static else w.attn)(splits * T * H * lora, splits * T * H * 4)   # a reference and a sum for each half of the columns
     _LAUNCHES += 2 if splits > 1 else 1
     return _C.mla_decode(q_abs, q_pe, latent_cache, md.query_start_loc, md.seq_lens, md.block_table, scale, max(ql), splits, ws_o, ws_ml, cos_sin,
-                         interleaved, fine, skip_min_len, sinks, gate)
+                         interleaved, fine, skip_min_len, sinks, gate, wide)
 
 
 MLA_PREFILL_MIN_LEN = 64           # portions of at least this many tokens attend in the expanded form

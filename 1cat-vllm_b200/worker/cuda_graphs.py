@@ -75,21 +75,22 @@ class DecodeGraphs:
         self.hits = self.misses = 0
 
     def plan(self, R: int, q: int, max_seq: int) -> Optional[tuple]:
-        """Returns (padded R, q, splits) or None when the batch must run eagerly."""
+        """Returns (padded R, q, splits) or None when the batch must run eagerly. Latent attention: (splits, whether the tcgen05 kernel runs)."""
         if not self.eligible or R > self.sizes[-1] or q > self.max_q:
             return None
         rp = self.sizes[bisect.bisect_left(self.sizes, R)]
         if self.own_plans:
             return rp, q, self._context_bucket(max_seq)
-        from onecat_vllm.ops.cuda import _sms, choose_decode_splits, plan_mla_splits
-        if self.geom[0] == "mla":
-            want = plan_mla_splits(self.geom[1], self.geom[2], [q] * rp, [max_seq], _sms(self.r.device), self.mla_wide)
+        from onecat_vllm.ops.cuda import _sms, choose_decode_splits, plan_mla
+        mla = self.geom[0] == "mla"
+        if mla:
+            want, wide = plan_mla(self.geom[1], self.geom[2], [q] * rp, [max_seq], _sms(self.r.device), self.mla_wide)
         else:
             want = choose_decode_splits(rp * self.geom[1], max_seq, _sms(self.r.device))
         s = 1  # bucketed to powers of two (rounding up keeps the grid sized for the live context)
         while s < want:
             s *= 2
-        return rp, q, min(s, 32)
+        return rp, q, (min(s, 32), wide) if mla else min(s, 32)
 
     def _context_bucket(self, max_seq: int) -> int:
         """Power of two of at least 512 that covers the keys a decode row walks (contexts beyond every layer's window share one bucket)."""
@@ -159,9 +160,14 @@ class DecodeGraphs:
         r.np_pack[o["slot"][0]: o["slot"][0] + o["slot"][1]] = -1
         r.d_pack.copy_(r.h_pack)
         r.d_bt.copy_(r.h_bt)
-        first = self._context_bucket(self.max_span or 1) if self.own_plans else 1
         for s in reversed(self.sizes):
-            self.capture((s, 1, first))
+            if self.own_plans:
+                self.capture((s, 1, self._context_bucket(self.max_span or 1)))
+            elif self.geom[0] == "mla":   # of short contexts and of longer ones
+                for key in dict.fromkeys([self.plan(s, 1, 1), (s, 1, (1, self.mla_wide))]):
+                    self.capture(key)
+            else:
+                self.capture((s, 1, 1))
         log.info_once(f"captured {len(self.graphs)} decode graphs (sizes up to {self.sizes[-1]})")
 
     def run(self, key: tuple, T: int) -> torch.Tensor:

@@ -45,7 +45,7 @@ def test_rope_and_cache_in_wide_accesses(T, Hq, Hkv, D, rot, norm, fp8):
 
 
 @pytest.mark.parametrize("qlens,ctxs,H,rope,options", [([1, 1, 1], [0, 62, 63], 64, 64, False), ([1, 1], [16, 5000], 128, 64, True), ([1, 2, 5], [0, 127, 300], 64, 32, True),
-                                                      ([3, 1, 0, 2], [77, 1, 9, 640], 24, 48, False), ([1] * 40, [130] * 40, 128, 64, False)])
+                                                      ([3, 1, 0, 2], [77, 1, 9, 640], 24, 48, False), ([1] * 40, [130] * 40, 128, 64, False), ([1] * 80, [61, 63, 64, 5] * 20, 16, 64, True)])
 def test_mla_decode_tiles_of_128_rows(qlens, ctxs, H, rope, options):
     """Contexts of one key to many tiles, tiles and pages that end with the context, rows that end inside a tile, several tokens a request, key
     parts below 64; the slots past a context hold NaN. Sinks and gates where asked. Weights and queries are bf16: 2^-8 each."""
@@ -97,7 +97,7 @@ def _mla_case(qlens, seq, H, g, q_pe, k_pe, lora=512, rope=64, bs=16):
 
 
 def _in_splits(md, H, splits):
-    md.static_ws, md.attn_plan = True, (("mla", H, 512), (md.max_query_len, 0, splits))
+    md.static_ws, md.attn_plan = True, (("mla", H, 512), (md.max_query_len, 0, (splits, True)))
     return md
 
 

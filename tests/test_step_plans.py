@@ -22,7 +22,18 @@ def test_latent_attention_is_split_for_the_kernel_that_runs(form, wide, monkeypa
     H, R, ctx = 16, 32, 4096
     per_sm = max(1, min(4, (227 << 10) // ((16 + 2 * 64) * (f["lora"] + 64) * 2 + 6144)))
     want = K.choose_decode_splits(2 * R, ctx, 148, 1, start=6.0, tile=1.3) if wide else K.choose_decode_splits(R, ctx, 148, per_sm)
-    assert K.plan_mla_splits(H, f["lora"], [1] * R, [ctx], 148, K.mla_decode_wide(**f)) == want
+    assert K.plan_mla(H, f["lora"], [1] * R, [ctx], 148, K.mla_decode_wide(**f)) == (want, wide)
     monkeypatch.setattr(K, "_sms", lambda device: 148)
     graphs = SimpleNamespace(eligible=True, sizes=[R], max_q=1, own_plans=False, geom=("mla", H, f["lora"]), mla_wide=wide, r=SimpleNamespace(device=None))
-    assert DecodeGraphs.plan(graphs, R, 1, ctx) == (R, 1, 1 << (want - 1).bit_length())
+    assert DecodeGraphs.plan(graphs, R, 1, ctx) == (R, 1, (1 << (want - 1).bit_length(), wide))
+
+
+@pytest.mark.parametrize("H,R,ctx,wide", [(16, 74, 16, True), (16, 75, 64, False), (16, 148, 190, False), (16, 149, 64, False), (16, 149, 100, True), (16, 256, 64, False),
+                                          (16, 400, 400, True), (8, 128, 256, False), (8, 200, 190, True), (8, 256, 1000, True), (17, 256, 64, True), (128, 400, 64, True)])
+def test_latent_rows_of_one_narrow_tile_and_short_contexts(H, R, ctx, wide):
+    """Requests of at most 16 rows run in tiles of 16 where tiles of 128 (two CTAs each) are more waves and the contexts short: measured on either side of the line."""
+    from onecat_vllm.ops import cuda as K
+    splits, chosen = K.plan_mla(H, 512, [1] * R, [ctx], 148, True)
+    assert chosen == wide and K.plan_mla(H, 512, [1] * R, [ctx], 148, False)[1] is False
+    if not wide:
+        assert splits == 1
