@@ -506,17 +506,50 @@ def choose_decode_splits(base_ctas: int, max_seq: int, num_sms: int, per_sm: int
     B200 (64 requests x 8 KV heads x 1150 keys): 71.7 us unsplit against 80.9 us in two splits, whose 1024 CTAs need four waves
     of 296 where 512 need two; 16 requests x 4096 keys: 66 us in two splits (one wave) against 83 us in three (two waves)."""
     nt = max(1, -(-max_seq // 64))
-    slots = per_sm * num_sms
     best, best_cost = 1, None
     for s in range(1, min(32, nt) + 1):
-        per = -(-nt // s)
-        if s > 1 and per < 2:
+        if s > 1 and -(-nt // s) < 2:
             break
-        waves = -(-(max(base_ctas, 1) * s) // slots)
-        cost = waves * (start + tile * per) + (6.0 + 0.15 * s if s > 1 else 0.0)  # the combine kernel reads one partial per split
+        cost = _split_cost(s, base_ctas, nt, per_sm * num_sms, start, tile)
         if best_cost is None or cost < best_cost - 1e-9:
             best, best_cost = s, cost
     return best
+
+
+def _split_cost(s: int, base_ctas: int, nt: int, slots: int, start: float, tile: float) -> float:
+    waves = -(-(max(base_ctas, 1) * s) // slots)
+    return waves * (start + tile * -(-nt // s)) + (6.0 + 0.15 * s if s > 1 else 0.0)  # the combine kernel reads one partial per split
+
+
+def decode_cost(D: int, rows: int, fp8: bool) -> dict:
+    """What a wave of the paged decode kernel costs, as arguments of ``choose_decode_splits``; ``rows``: query tokens x heads of a group. Over an
+    fp8 cache (attention_fp8.cu) three CTAs fit an SM with heads of 128 and up to 16 rows, else two; times measured with full SMs."""
+    return dict(per_sm=3 if D == 128 and rows <= 16 else 2, start=5.0, tile=1.35) if fp8 and D >= 128 else {}
+
+
+def choose_graph_splits(base_ctas: int, max_seq: int, num_sms: int, D: int, rows: int, fp8: bool) -> int:
+    """Splits of a captured decode graph: a power of two, so that few graphs are captured. Over an fp8 cache a doubling has to win by 7 % in the
+    cost model (less is within its error); rounding the best number up would cross into another wave: 16 requests x 2000 keys x 8 heads 34 us
+    in two splits, 36 in four (best: three, 32); 32 x 4096 90 / 91 / 83 / 94 in one, two, four, eight."""
+    cost = decode_cost(D, rows, fp8)
+    s = 1
+    if not cost:
+        want = choose_decode_splits(base_ctas, max_seq, num_sms)
+        while s < want:
+            s *= 2
+        return min(s, 32)
+    nt, args = max(1, -(-max_seq // 64)), (cost["per_sm"] * num_sms, cost["start"], cost["tile"])
+    best = _split_cost(1, base_ctas, nt, *args)
+    for n in (2, 4, 8, 16, 32):
+        c = _split_cost(n, base_ctas, nt, *args)
+        if -(-nt // n) >= 2 and c < 0.93 * best:
+            s, best = n, c
+    return s
+
+
+def attn_plan_key(Hq: int, Hkv: int, D: int, fp8: bool) -> tuple:
+    """What a step's ``attn_plan`` was made for: layers of another geometry or cache type plan anew."""
+    return (Hq, Hkv, D, "fp8") if fp8 else (Hq, Hkv, D)
 
 
 def plan_attention(query_lens: list, seq_lens: list, Hq: int, Hkv: int, D: int, num_sms: int, force_splits: int = 0, span: int = 0,
@@ -537,8 +570,7 @@ def plan_attention(query_lens: list, seq_lens: list, Hq: int, Hkv: int, D: int, 
     if n_short:
         max_s = max((s for q, s in zip(query_lens, seq_lens) if q <= short), default=1)
         per_sm = {64: 5, 128: 4}.get(D, 2) if extended and short * G <= 16 else 2
-        # attention_fp8.cu: three CTAs per SM for heads of 128, two for 256; its times measured with full SMs
-        cost = dict(per_sm=3 if D == 128 and short * G <= 16 else 2, start=5.0, tile=1.35) if fp8 and D >= 128 else dict(per_sm=per_sm)
+        cost = decode_cost(D, short * G, fp8) or dict(per_sm=per_sm)
         splits = choose_decode_splits(n_short * Hkv, min(max_s, span) if span else max_s, num_sms, **cost)
     if force_splits:
         splits = force_splits
@@ -567,11 +599,12 @@ def paged_attention(q, kv_cache, md, scale, out=None, lse=None, window=0, softca
         _LAUNCHES += 1
         return out
     extended = keep > 0 or bias_table is not None or gate is not None or kv_cache.shape[1] == 1 or chunk > 0
-    key = (Hq, Hkv, D, attention_span(min(window, chunk) if window and chunk else window or chunk, keep)) if extended else (Hq, Hkv, D)
+    fp8 = kv_cache.dtype == torch.float8_e4m3fn
+    key = (Hq, Hkv, D, attention_span(min(window, chunk) if window and chunk else window or chunk, keep)) if extended else attn_plan_key(Hq, Hkv, D, fp8)
     plan = getattr(md, "attn_plan", None)
     if plan is None or plan[0] != key:
         plan = (key, plan_attention(md.query_lens_cpu, md.seq_lens_cpu, Hq, Hkv, D, _sms(q.device), span=key[3] if extended else 0,
-                                    extended=kv_cache.shape[1] == 1, fp8=kv_cache.dtype == torch.float8_e4m3fn))
+                                    extended=kv_cache.shape[1] == 1, fp8=fp8))
         md.attn_plan = plan
     short, tiles, splits = plan[1]
     n_short = sum(1 for x in md.query_lens_cpu if 0 < x <= short)

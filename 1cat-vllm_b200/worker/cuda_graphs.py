@@ -52,6 +52,7 @@ class DecodeGraphs:
         if layers:
             a = layers[0].self_attn
             self.geom = (a.Hq, a.Hkv, a.D)
+            self.kv_fp8 = runner._attn_kv_dtype() == torch.float8_e4m3fn
             K.workspace(runner.device).attn_static(32 * tmax * max(a.Hq * a.D for a in attns), 32 * tmax * 2 * max(a.Hq for a in attns))
             for a in mlas:
                 K.workspace(runner.device).attn_static(32 * tmax * a.H * a.lora_pad, 32 * tmax * a.H * 4)
@@ -81,16 +82,15 @@ class DecodeGraphs:
         rp = self.sizes[bisect.bisect_left(self.sizes, R)]
         if self.own_plans:
             return rp, q, self._context_bucket(max_seq)
-        from onecat_vllm.ops.cuda import _sms, choose_decode_splits, plan_mla
-        mla = self.geom[0] == "mla"
-        if mla:
-            want, wide = plan_mla(self.geom[1], self.geom[2], [q] * rp, [max_seq], _sms(self.r.device), self.mla_wide)
-        else:
-            want = choose_decode_splits(rp * self.geom[1], max_seq, _sms(self.r.device))
+        from onecat_vllm.ops.cuda import _sms, choose_graph_splits, plan_mla
+        if self.geom[0] != "mla":
+            Hq, Hkv, D = self.geom
+            return rp, q, choose_graph_splits(rp * Hkv, max_seq, _sms(self.r.device), D, q * (Hq // Hkv), self.kv_fp8)
+        want, wide = plan_mla(self.geom[1], self.geom[2], [q] * rp, [max_seq], _sms(self.r.device), self.mla_wide)
         s = 1  # bucketed to powers of two (rounding up keeps the grid sized for the live context)
         while s < want:
             s *= 2
-        return rp, q, (min(s, 32), wide) if mla else min(s, 32)
+        return rp, q, (min(s, 32), wide)
 
     def _context_bucket(self, max_seq: int) -> int:
         """Power of two of at least 512 that covers the keys a decode row walks (contexts beyond every layer's window share one bucket)."""
@@ -115,11 +115,12 @@ class DecodeGraphs:
         elif self.geom[0] == "mla":
             md.attn_plan = (self.geom, (q, 0, splits))
         else:
+            from onecat_vllm.ops.cuda import attn_plan_key
             Hq, Hkv, D = self.geom
             G = Hq // Hkv
             short = (32 if D == 128 else 16) // G
             # uniform batch: every request has q tokens; they take the decode kernel when q*G rows fit its tile
-            md.attn_plan = ((Hq, Hkv, D), (q if q <= short else short, 0 if q <= short else rp * (-(-q // (64 // G))), splits))
+            md.attn_plan = (attn_plan_key(Hq, Hkv, D, self.kv_fp8), (q if q <= short else short, 0 if q <= short else rp * (-(-q // (64 // G))), splits))
         md.static_ws = True
         return md
 

@@ -218,7 +218,7 @@ def test_decode_over_an_fp8_cache(D, Hq, Hkv, qlens, ctxs, options):
     for splits in (1, 3, None):
         md = AttentionMetadata(R, T, qsl.cuda(), sl.cuda(), bt.cuda(), None, None, max(qlens), max(seq), query_lens_cpu=list(qlens), seq_lens_cpu=seq)
         if splits:
-            md.attn_plan = ((Hq, Hkv, D), (max(qlens), 0, splits))
+            md.attn_plan = (K().attn_plan_key(Hq, Hkv, D, True), (max(qlens), 0, splits))
         out = K().paged_attention(q.cuda(), cache.cuda(), md, D ** -0.5, window=window, softcap=softcap, sinks=None if sinks is None else sinks.cuda())
         assert K().check_status() == 0
         _close(out, want, 2e-2, 1e-2, f"{splits} splits")

@@ -37,3 +37,19 @@ def test_latent_rows_of_one_narrow_tile_and_short_contexts(H, R, ctx, wide):
     assert chosen == wide and K.plan_mla(H, 512, [1] * R, [ctx], 148, False)[1] is False
     if not wide:
         assert splits == 1
+
+
+@pytest.mark.parametrize("R,ctx,Hkv,D,best,slower", [(8, 1152, 8, 128, 4, 8), (16, 2000, 8, 128, 2, 4), (64, 1152, 8, 128, 1, 4), (128, 1152, 8, 128, 1, 2), (32, 4096, 8, 128, 1, 8), (64, 2300, 8, 128, 2, 4),
+                                                     (8, 32768, 8, 128, 16, 8), (32, 500, 4, 128, 1, 2), (256, 1152, 4, 256, 1, 2), (8, 32768, 4, 256, 8, 4), (1, 4000, 8, 128, 16, 4)])
+def test_captured_decoding_over_an_fp8_cache_is_split_for_its_kernel(R, ctx, Hkv, D, best, slower, monkeypatch):
+    """Graphs and eager steps take their costs from one place; ``slower``: a number of splits that was measured slower than the chosen one."""
+    from types import SimpleNamespace
+    from onecat_vllm.ops import cuda as K
+    from onecat_vllm.worker.cuda_graphs import DecodeGraphs
+    monkeypatch.setattr(K, "_sms", lambda device: 148)
+    graphs = lambda fp8: SimpleNamespace(eligible=True, sizes=[R], max_q=1, own_plans=False, geom=(5 * Hkv, Hkv, D), kv_fp8=fp8, r=SimpleNamespace(device=None))
+    assert DecodeGraphs.plan(graphs(True), R, 1, ctx) == (R, 1, best) != (R, 1, slower)
+    want = K.choose_decode_splits(R * Hkv, ctx, 148)
+    assert DecodeGraphs.plan(graphs(False), R, 1, ctx) == (R, 1, min(32, 1 << (want - 1).bit_length()))
+    assert K.plan_attention([1] * R, [ctx] * R, 5 * Hkv, Hkv, D, 148, fp8=True)[2] == K.choose_decode_splits(R * Hkv, ctx, 148, **K.decode_cost(D, 5, True))
+    assert len({K.attn_plan_key(5 * Hkv, Hkv, D, f) for f in (True, False)}) == 2
