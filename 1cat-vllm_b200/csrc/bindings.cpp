@@ -25,6 +25,31 @@ void check_bf16(const torch::Tensor& t, const char* name) {
   TORCH_CHECK(t.scalar_type() == torch::kBFloat16, name, " must be bf16");
 }
 
+// The kernels of a dense product: a few tokens (gemm_skinny.cu), packed weights widened in slabs and bf16 weights over pairs of SMs (gemm_pair.cu),
+// tiles of one SM (gemm_sm100.cu).
+enum class GemmRoute { kTiles, kSkinny, kWiden, kPair };
+GemmRoute gemm_route(const oc::GemmParams& p, int sms) {
+  if (oc::gemm_skinny_takes(p, sms)) return GemmRoute::kSkinny;
+  if (oc::gemm_widen_takes(p, sms)) return GemmRoute::kWiden;
+  return p.w4 == nullptr && oc::gemm_pair_takes(p, sms) ? GemmRoute::kPair : GemmRoute::kTiles;
+}
+
+// (kernel, slabs) that a product of this form takes on a device with so many SMs; wkind 0: bf16 weights.
+std::tuple<std::string, int64_t> gemm_route_of(int64_t T, int64_t n_rows, int64_t K, int64_t wkind, int64_t epi, bool f32_out, int64_t sms) {
+  oc::GemmParams p{};
+  p.T = (int)T; p.N = p.n_rows = (int)n_rows; p.n_out = (int)n_rows / 2; p.K = (int)K; p.epi = (int)epi; p.wkind = (int)wkind;
+  // only whether they are there is looked at
+  p.w4 = wkind != 0 ? reinterpret_cast<const uint8_t*>(&p) : nullptr;
+  if (f32_out) p.out_f32 = reinterpret_cast<float*>(&p);
+  else p.out = reinterpret_cast<__nv_bfloat16*>(&p);
+  switch (gemm_route(p, (int)sms)) {
+    case GemmRoute::kSkinny: return {"skinny", 0};
+    case GemmRoute::kWiden: { const int64_t rows = oc::gemm_widen_rows(p, (int)sms); return {"widen", (n_rows + rows - 1) / rows}; }
+    case GemmRoute::kPair: return {"pair", 0};
+    default: return {"tiles", 0};
+  }
+}
+
 // out[T, n_out or N] = epilogue(X[T,K] @ W^T). Exactly one of `w` (bf16 [n_rows, K]) and `w4` (packed tiles) is given.
 void gemm(torch::Tensor x, c10::optional<torch::Tensor> w, c10::optional<torch::Tensor> w4, c10::optional<torch::Tensor> w4_sz,
           torch::Tensor out, c10::optional<torch::Tensor> bias, torch::Tensor ws, torch::Tensor counters, int64_t N, int64_t n_rows,
@@ -91,18 +116,19 @@ void gemm(torch::Tensor x, c10::optional<torch::Tensor> w, c10::optional<torch::
   p.trace = (unsigned long long*)(uintptr_t)trace_ptr;
   p.push_sel = (const int*)(uintptr_t)push_sel;
   p.push_sel_stride = (long long)push_sel_stride;
-  if (force_splits <= 0 && force_tn <= 0 && oc::gemm_skinny_takes(p)) {
+  const GemmRoute route = force_splits <= 0 && force_tn <= 0 ? gemm_route(p, sm_count()) : GemmRoute::kTiles;
+  if (route == GemmRoute::kSkinny) {
     const int rc = oc::gemm_skinny_launch(p, x.data_ptr(), (int)x.stride(0), sm_count(), cur_stream());
     TORCH_CHECK(rc == 0, "gemm launch failed with code ", rc);
     return;
   }
-  if (force_splits <= 0 && force_tn <= 0 && oc::gemm_widen_takes(p, sm_count())) {
+  if (route == GemmRoute::kWiden) {
     auto slab = torch::empty({oc::gemm_widen_rows(p, sm_count()), p.K}, x.options());
     const int rc = oc::gemm_widen_launch(p, x.data_ptr(), (int)x.stride(0), slab.data_ptr(), sm_count(), cur_stream());
     TORCH_CHECK(rc == 0, "gemm launch failed with code ", rc);
     return;
   }
-  if (force_splits <= 0 && force_tn <= 0 && !w4.has_value() && oc::gemm_pair_takes(p, sm_count())) {
+  if (route == GemmRoute::kPair) {
     const int rc = oc::gemm_pair_launch(p, x.data_ptr(), (int)x.stride(0), wptr, ldw, sm_count(), cur_stream());
     TORCH_CHECK(rc == 0, "gemm launch failed with code ", rc);
     return;
@@ -1413,6 +1439,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("mla_decode", &mla_decode);
   m.def("mla_tensor_core_sizes", &mla_tensor_core_sizes);
   m.def("mla_decode_wide", &mla_decode_wide);
+  m.def("gemm_route", &gemm_route_of);
   m.def("mla_prepare", &mla_prepare);
   m.def("mla_prefill_inputs", &mla_prefill_inputs);
   m.def("mla_prefill", &mla_prefill);

@@ -275,17 +275,30 @@ int go(const GemmParams& p, const void* x, int ldx, int num_sms, cudaStream_t st
 }
 
 constexpr int kSkinnyTokens = 16;
-constexpr long long kSmallWeights = 32ll << 20;
+constexpr long long kSmallWeights = 32ll << 20, kFewWeights = 24ll << 20;
 
 }  // namespace
 
-// Which dense products take this kernel (both sides measured, us): int4 with up to eight tokens always (34816 x 5120: 46 to 49 against 54;
-// 5120 x 17408 in one CTA wave about equal, 40 against 38; 2048 x 1024: 8 against 15); up to sixteen tokens, and the kinds that take more
-// instructions to widen, while the weights are small, where this kernel's short start counts (fp8 11264 x 2048: 18 against 24, 34816 x 5120: 72
-// against 60; int4 at 16 tokens 18 against 22 and 61 against 54).
-bool gemm_skinny_takes(const GemmParams& p) {
-  return p.w4 != nullptr && p.n_push == 0 && p.out != nullptr && (p.epi == EPI_STORE || p.epi == EPI_SILU_MUL) &&
-         ((p.wkind == 1 && p.T <= 8) || (p.T <= kSkinnyTokens && (long long)p.n_rows * p.K <= kSmallWeights));
+// Which dense products take this kernel (us here / on the tcgen05 path of gemm_sm100.cu, which splits k over clusters and starts slower).
+// Up to 32 M weights, where its short start counts: 2048 x 1024 8 / 15, 4096 x 4096 int4 and MXFP4 12 / 20, fp8 14 / 20. The kinds that take more
+// instructions to widen stop earlier: the fp4 kinds beyond eight tokens at 24 M (5120 x 5120 22.5 / 22, 16384 x 1536 18 / 20.5), fp8 at 24 M (5120 x
+// 5120 24.5 / 23 for one token, 28 / 24 for twelve; 12288 x 2048 18.5 / 23.5). fp8 also stops
+//   * where its CTAs leave three tenths of their waves' SMs idle and k is not short: 5120 x 4096, 160 CTAs, 22 / 21.5 for four tokens, 25 / 21.5 for
+//     nine (4096 x 5120, 128 CTAs: 16 / 22);
+//   * where long k meets few rows, a chain per warp: 1024 x 8192 20 / 19, 22 / 19 for nine tokens; 512 x 7168 18.4 / 17.4; 1536 x 7168 18 / 19 up to
+//     eight tokens, 20 / 19 above; 2048 x 8192 19 / 23.
+// Beyond 32 M int4 with up to eight tokens (34816 x 5120: 45 to 49 / 53; 8192 x 28672: 62 to 67 / 76), except where its CTAs leave two fifths of
+// their waves' SMs idle for long: 5120 x 17408, 160 CTAs, 41 / 39 for four tokens, 43 / 39 for eight, 5120 x 25600 52.5 / 50 for one (4800 x 8192
+// 23.6 / 25.8).
+bool gemm_skinny_takes(const GemmParams& p, int num_sms) {
+  if (p.w4 == nullptr || p.n_push != 0 || p.out == nullptr || (p.epi != EPI_STORE && p.epi != EPI_SILU_MUL) || p.T > kSkinnyTokens) return false;
+  const long long weights = (long long)p.n_rows * p.K;
+  const int ctas = (p.n_rows + 31) / 32, slots = (ctas + num_sms - 1) / num_sms * num_sms;
+  if (p.wkind == 2)
+    return weights <= kFewWeights && (p.K < 4096 || ctas <= num_sms || 10 * ctas >= 7 * slots) &&
+           (p.K <= 6144 || p.n_rows >= 2048 || (p.n_rows >= 1536 && p.T <= 8));
+  if (p.wkind != 1) return weights <= (p.T <= 8 ? kSmallWeights : kFewWeights);
+  return weights <= kSmallWeights || (p.T <= 8 && (p.K <= 8192 || 5 * ctas >= 3 * slots));
 }
 
 // Packed weights and up to 16 tokens; operands and results as in gemm_launch.

@@ -66,7 +66,7 @@ int gemm_widen_rows(const GemmParams& p, int num_sms);
 int gemm_widen_launch(const GemmParams& p, const void* x, int ldx, void* slab, int num_sms, cudaStream_t st);
 unsigned int* gemm_pair_status_word();
 // a few tokens, packed weights (gemm_skinny.cu)
-bool gemm_skinny_takes(const GemmParams& p);
+bool gemm_skinny_takes(const GemmParams& p, int num_sms);
 int gemm_skinny_launch(const GemmParams& p, const void* x, int ldx, int num_sms, cudaStream_t stream);
 unsigned int* gemm_status_word();
 int gemm_kernel_info(int wkind, int small, int smem, int out[6]);

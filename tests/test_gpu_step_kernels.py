@@ -169,7 +169,7 @@ def _packed(kind, N, Kd, g):
 
 
 @pytest.mark.parametrize("kind", [1, 2, 3, 4])
-@pytest.mark.parametrize("T,N,Kd,gated", [(1, 128, 128, False), (8, 160, 1152, True), (9, 96, 4224, False), (16, 5120, 704, True), (3, 224, 64, True), (13, 64, 8320, False)])
+@pytest.mark.parametrize("T,N,Kd,gated", [(1, 128, 128, False), (8, 160, 1152, True), (9, 96, 4224, False), (16, 5120, 704, True), (3, 224, 64, True), (13, 64, 8320, False), (13, 2080, 8320, False)])
 def test_gemm_of_a_few_tokens(kind, T, N, Kd, gated):
     """One and two blocks of eight tokens, full and ragged, rows that end inside a tile, k ranges of an odd number of tiles, of fewer than the warps
     and of many, gated and plain (with a bias) epilogues, a strided activation. Weights are rounded to bf16 where they are widened; fp32 sums, one rounding at the end."""

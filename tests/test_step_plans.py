@@ -53,3 +53,15 @@ def test_captured_decoding_over_an_fp8_cache_is_split_for_its_kernel(R, ctx, Hkv
     assert DecodeGraphs.plan(graphs(False), R, 1, ctx) == (R, 1, min(32, 1 << (want - 1).bit_length()))
     assert K.plan_attention([1] * R, [ctx] * R, 5 * Hkv, Hkv, D, 148, fp8=True)[2] == K.choose_decode_splits(R * Hkv, ctx, 148, **K.decode_cost(D, 5, True))
     assert len({K.attn_plan_key(5 * Hkv, Hkv, D, f) for f in (True, False)}) == 2
+
+
+@pytest.mark.parametrize("kind,N,Kd,T,skinny", [
+    (1, 2048, 1024, 16, True), (1, 5120, 5120, 16, True), (1, 34816, 5120, 8, True), (1, 34816, 5120, 9, False), (1, 8192, 28672, 8, True), (1, 5120, 17408, 1, False),
+    (1, 4800, 8192, 8, True), (1, 2048, 1024, 17, False), (2, 4096, 4096, 16, True), (2, 16384, 1536, 16, True), (2, 5120, 5120, 1, False), (2, 5120, 4096, 2, False),
+    (2, 4096, 5120, 16, True), (2, 1024, 8192, 1, False), (2, 2048, 8192, 16, True), (2, 1536, 7168, 8, True), (2, 1536, 7168, 9, False), (2, 2112, 7168, 16, True),
+    (2, 1024, 5120, 16, True), (3, 5120, 5120, 8, True), (3, 5120, 5120, 9, False), (4, 6144, 5120, 16, False), (4, 16384, 1536, 16, True), (3, 34816, 5120, 1, False)])
+def test_packed_products_of_a_few_tokens(kind, N, Kd, T, skinny):
+    """Either side of each line of the rule, as measured."""
+    from onecat_vllm.ops import _C
+    assert (_C.gemm_route(T, N, Kd, kind, 0, False, 148)[0] == "skinny") == skinny
+    assert _C.gemm_route(T, N, Kd, 0, 0, False, 148)[0] == "tiles"
