@@ -309,7 +309,8 @@ void paged_attention(torch::Tensor q, torch::Tensor kv_cache, torch::Tensor out,
   p.kv_fp8 = kv_cache.scalar_type() == torch::kFloat8_e4m3fn;
   p.k_scale = (float)k_scale;
   p.v_scale = (float)v_scale;
-  TORCH_CHECK(mode != 2 || !p.kv_fp8, "an fp8 KV cache runs on the mma.sync kernels");
+  const bool tc = mode == 2 || mode == 4;
+  TORCH_CHECK(!tc || !p.kv_fp8, "an fp8 KV cache runs on the mma.sync kernels");
   if (sinks.has_value()) {
     TORCH_CHECK(sinks->is_cuda() && sinks->scalar_type() == torch::kFloat32 && sinks->is_contiguous() && sinks->numel() == q.size(1),
                 "sinks must be a contiguous fp32 CUDA tensor with one entry per query head");
@@ -331,7 +332,7 @@ void paged_attention(torch::Tensor q, torch::Tensor kv_cache, torch::Tensor out,
   }
   p.chunk = (int)chunk;
   const bool extended = chunk > 0 || keep > 0 || p.kv_shared || p.bias != nullptr || p.gate != nullptr;
-  TORCH_CHECK(mode != 2 || (window == 0 && softcap == 0.0 && !sinks.has_value() && !extended), "window / softcap / sinks and the like run on the mma.sync kernels");
+  TORCH_CHECK(!tc || (window == 0 && softcap == 0.0 && !sinks.has_value() && !extended), "window / softcap / sinks and the like run on the mma.sync kernels");
   TORCH_CHECK(!(extended && p.kv_fp8), "an fp8 KV cache has no distance bias, kept tokens, output gate or shared keys and values");
   if (mode == 1 && splits > 1) {
     TORCH_CHECK(ws_o.has_value() && ws_ml.has_value(), "split-KV needs workspaces");
@@ -341,8 +342,9 @@ void paged_attention(torch::Tensor q, torch::Tensor kv_cache, torch::Tensor out,
     p.ws_ml = ws_ml->data_ptr<float>();
   }
   if (p.T == 0 || p.R == 0) return;
-  // mode 0: mma.sync prefill, 1: decode / short verify queries, 2: tcgen05 prefill (D = 128, query tiles of 128 tokens), 3: fp32
-  int rc = mode == 3 ? oc::attention_f32_launch(p, false, cur_stream()) : mode == 2 ? oc::attention_prefill_tc_launch(p, kv_cache.size(0), cur_stream()) : oc::attention_launch(p, (int)mode, cur_stream());
+  // mode 0: mma.sync prefill, 1: decode / short verify queries, 2: tcgen05 prefill (D = 128, 256 query tokens a CTA), 3: fp32,
+  // 4: tcgen05 prefill of short contexts (128 query tokens a CTA)
+  int rc = mode == 3 ? oc::attention_f32_launch(p, false, cur_stream()) : tc ? oc::attention_prefill_tc_launch(p, kv_cache.size(0), mode == 2, cur_stream()) : oc::attention_launch(p, (int)mode, cur_stream());
   TORCH_CHECK(rc == 0, "attention launch failed with code ", rc);
 }
 

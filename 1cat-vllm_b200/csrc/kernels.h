@@ -157,8 +157,8 @@ bool diff_prefill_tc_sizes(int D, float softcap);
 int diff_prefill_tc_launch(const AttnParams& p, long long num_blocks, cudaStream_t st);
 unsigned int* diff_prefill_status_word();
 
-// tcgen05 prefill (attention_tc.cu): D == 128, 128-token query tiles; num_q_tiles counts those tiles.
-int attention_prefill_tc_launch(const AttnParams& p, long long num_blocks, cudaStream_t st);
+// tcgen05 prefill (attention_tc.cu): D == 128; num_q_tiles counts pieces of 256 query tokens (pairs of tiles) or single tiles of 128.
+int attention_prefill_tc_launch(const AttnParams& p, long long num_blocks, bool pairs, cudaStream_t st);
 unsigned int* attention_tc_status_word();
 
 

@@ -582,6 +582,24 @@ def attention_span(window: int, keep: int) -> int:
     return 64 * (-(-window // 64) + 1 + -(-keep // 64)) if window else 0
 
 
+def prompt_tiles(query_lens: list, seq_lens: list, short: int, heads: int, num_sms: int) -> tuple[bool, int]:
+    """(whether a CTA of the tcgen05 prompt kernel takes 256 query tokens, pieces) of a step's portions longer than ``short``. Two tiles of 128 in
+    turn on the tensor core are the faster form, except for short contexts, where a CTA's chain of waits counts (us, single / pairs):
+
+    * all single tiles in one wave of CTAs and up to six key tiles (three, where no portion has a second query tile): 16 heads, 256 tokens
+      14.3 / 18.4, 512 20.5 / 22.5, 700 24.6 / 24.8; 40 heads, 300 tokens 16.6 / 18.4, 512 tokens (two waves) 28.7 / 24.6; 4 heads, a portion
+      of 128 over 400 keys 22.5 / 21.0;
+    * portions of single tiles and up to three key tiles: 40 heads, 32 x 128 tokens 86 / 92.5, 128 x 40 375 / 389, 8 x 128 over 200 keys 43 / 45, 32 x 128 over
+      500 keys 172 / 166; with fewer than 16 heads the other way, 8 heads, 128 x 40 tokens 88 / 84."""
+    portions = [(n, s) for n, s in zip(query_lens, seq_lens) if n > short]
+    single, pairs = (sum(-(-n // t) for n, _ in portions) for t in (128, 256))
+    keys = -(-max(s for _, s in portions) // 128)   # captured graphs know no lengths: 0
+    alone = max(n for n, _ in portions) <= 128
+    if 0 < keys <= 3 and alone and heads >= 16 or 0 < keys <= (3 if alone else 6) and single * heads <= num_sms:
+        return False, single
+    return True, pairs
+
+
 def paged_attention(q, kv_cache, md, scale, out=None, lse=None, window=0, softcap=0.0, sinks=None, keep=0, bias_table=None, gate=None, chunk=0):
     """``window`` (tokens, 0 = full), ``softcap`` (0 = off), ``sinks`` (fp32 ``[Hq]``), ``keep`` (first tokens visible outside the window),
     ``bias_table`` (fp32 ``[Hq, n]`` by distance), ``gate`` (``[T, Hq]`` logits), ``chunk`` (positions, 0 = off) and a cache with one tensor per page select the mma.sync
@@ -619,9 +637,8 @@ def paged_attention(q, kv_cache, md, scale, out=None, lse=None, window=0, softca
     if tiles:
         if (D == 128 and q.stride(1) == D and _ATTN_PREFILL_TC and scale > 0 and not window and not softcap and sinks is None and not extended
                 and kv_cache.dtype == torch.bfloat16):
-            # tcgen05 kernel: 256 query tokens per CTA
-            tiles_tc = sum(-(-x // 256) for x in md.query_lens_cpu if x > short)
-            _C.paged_attention(q, kv_cache, out, lse, md.query_start_loc, md.seq_lens, md.block_table, scale, 2, tiles_tc, 1,
+            pairs, tiles_tc = prompt_tiles(md.query_lens_cpu, md.seq_lens_cpu, short, Hq, _sms(q.device))
+            _C.paged_attention(q, kv_cache, out, lse, md.query_start_loc, md.seq_lens, md.block_table, scale, 2 if pairs else 4, tiles_tc, 1,
                                md.max_query_len, short, None, None, 0, 0.0, None, 1.0, 1.0)
         else:
             _C.paged_attention(q, kv_cache, out, lse, md.query_start_loc, md.seq_lens, md.block_table, scale, 0, tiles, 1,

@@ -224,10 +224,15 @@ def test_decode_over_an_fp8_cache(D, Hq, Hkv, qlens, ctxs, options):
         _close(out, want, 2e-2, 1e-2, f"{splits} splits")
 
 
-@pytest.mark.parametrize("qlens,ctxs,Hq,Hkv,scale", [([256, 257, 1, 128], [0, 1, 500, 128], 8, 2, 1.0), ([129, 640, 17], [127, 300, 2000], 4, 4, 1.0), ([700], [0], 2, 1, 30.0)])
-def test_prompt_attention_in_pairs_of_query_tiles(qlens, ctxs, Hq, Hkv, scale):
+@pytest.mark.parametrize("qlens,ctxs,Hq,Hkv,scale", [([256, 257, 1, 128], [0, 1, 500, 128], 8, 2, 1.0), ([129, 640, 17], [127, 300, 2000], 4, 4, 1.0), ([700], [0], 2, 1, 30.0),
+                                                        ([128, 17, 1, 100], [0, 239, 500, 256], 16, 2, 1.0), ([129, 400], [300, 0], 8, 2, 1.0), ([700], [60], 2, 1, 30.0)])
+@pytest.mark.parametrize("pairs", [None, True, False])
+def test_prompt_attention_in_pairs_of_query_tiles(qlens, ctxs, Hq, Hkv, scale, pairs, monkeypatch):
     """Portions that end inside the first or the second tile of a pair, one that fills both, tiles of unequal numbers of key tiles, a decoding request
-    beside them, and scores that grow by far more than 2^8 along a row (the accumulator is rescaled). Weights are bf16 (2^-8)."""
+    beside them, and scores that grow by far more than 2^8 along a row (the accumulator is rescaled). As planned, and each form
+    (pairs, single tiles) for all of them. Weights are bf16 (2^-8)."""
+    if pairs is not None:
+        monkeypatch.setattr(K(), "prompt_tiles", lambda ql, sl, short, heads, sms: (pairs, sum(-(-n // (256 if pairs else 128)) for n in ql if n > short)))
     from onecat_vllm.worker.attn_metadata import AttentionMetadata
     D, bs, R, T = 128, 16, len(qlens), sum(qlens)
     g = torch.Generator().manual_seed(T)

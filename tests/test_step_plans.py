@@ -65,3 +65,16 @@ def test_packed_products_of_a_few_tokens(kind, N, Kd, T, skinny):
     from onecat_vllm.ops import _C
     assert (_C.gemm_route(T, N, Kd, kind, 0, False, 148)[0] == "skinny") == skinny
     assert _C.gemm_route(T, N, Kd, 0, 0, False, 148)[0] == "tiles"
+
+
+@pytest.mark.parametrize("n,q,ctx,heads,pairs", [
+    (1, 64, 0, 40, False), (1, 256, 0, 16, False), (1, 300, 0, 40, False), (1, 512, 0, 16, False), (1, 512, 0, 40, True), (1, 1024, 0, 8, True), (1, 128, 400, 4, True),
+    (16, 256, 0, 4, False), (16, 512, 0, 4, True), (32, 128, 0, 40, False), (8, 128, 200, 40, False), (32, 128, 500, 40, True), (128, 40, 0, 8, True), (32, 128, 0, 4, False),
+    (4, 200, 0, 40, True), (1, 8192, 0, 40, True), (1, 64, 4000, 40, True)])
+def test_prompt_attention_takes_single_tiles_for_short_contexts(n, q, ctx, heads, pairs):
+    """Either side of the lines of the rule, as measured; decoding requests beside the portions do not count, and unknown lengths (a graph) take pairs."""
+    from onecat_vllm.ops import cuda as K
+    tiles = n * -(-q // (256 if pairs else 128))
+    assert K.prompt_tiles([q] * n, [q + ctx] * n, 6, heads, 148) == (pairs, tiles)
+    assert K.prompt_tiles([1, 6] + [q] * n, [9000, 9000] + [q + ctx] * n, 6, heads, 148) == (pairs, tiles)
+    assert K.prompt_tiles([q] * n, [0] * n, 6, heads, 148) == (True, n * -(-q // 256))
