@@ -48,7 +48,7 @@ def test_rope_and_cache_in_wide_accesses(T, Hq, Hkv, D, rot, norm, fp8):
                                                       ([3, 1, 0, 2], [77, 1, 9, 640], 24, 48, False), ([1] * 40, [130] * 40, 128, 64, False), ([1] * 80, [61, 63, 64, 5] * 20, 16, 64, True)])
 def test_mla_decode_tiles_of_128_rows(qlens, ctxs, H, rope, options):
     """Contexts of one key to many tiles, tiles and pages that end with the context, rows that end inside a tile, several tokens a request, key
-    parts below 64; the slots past a context hold NaN. Sinks and gates where asked. Weights and queries are bf16: 2^-8 each."""
+    parts below 64, and requests of 16 rows that stay with the 16-row kernel; the slots past a context hold NaN. Sinks and gates where asked. Weights and queries are bf16: 2^-8 each."""
     from onecat_vllm.worker.attn_metadata import AttentionMetadata
     lora, bs, R, T = 512, 16, len(qlens), sum(qlens)
     g = torch.Generator().manual_seed(T + H)
@@ -150,20 +150,20 @@ def _packed(kind, N, Kd, g):
     """(packed tiles, scale table, padded rows, k tiles per group, weights in fp64) of random weights."""
     n = 64 if Kd % 128 else 128   # group
     if kind == 1:
-        q, z = torch.randint(0, 16, (N, Kd), generator=g, dtype=torch.uint8), torch.randint(0, 16, (N, Kd // n), generator=g, dtype=torch.uint8)
-        s = torch.rand(N, Kd // n, generator=g) * 0.01 + 0.001
+        q, z = torch.randint(0, 16, (N, Kd), generator=g, dtype=torch.uint8, device=g.device), torch.randint(0, 16, (N, Kd // n), generator=g, dtype=torch.uint8, device=g.device)
+        s = torch.rand(N, Kd // n, generator=g, device=g.device) * 0.01 + 0.001
         w = ((q.float() - z.float().repeat_interleave(n, 1)) * s.bfloat16().float().repeat_interleave(n, 1)).bfloat16().double()
         return (*K().pack_w4(q.cuda(), z.cuda(), s.cuda(), n), n // 64, w)
     if kind == 2:
-        c = torch.randn(N, Kd, generator=g).to(torch.float8_e4m3fn)
-        s = torch.rand(N, Kd // n, generator=g) * 0.02 + 0.001
+        c = torch.randn(N, Kd, generator=g, device=g.device).to(torch.float8_e4m3fn)
+        s = torch.rand(N, Kd // n, generator=g, device=g.device) * 0.02 + 0.001
         return (*K().pack_fp8(c.view(torch.uint8).cuda(), s.cuda(), n), n // 64, (c.float() * s.bfloat16().float().repeat_interleave(n, 1)).bfloat16().double())
-    c = torch.randint(0, 256, (N, Kd // 2), generator=g, dtype=torch.uint8)
-    values = torch.tensor([0, .5, 1, 1.5, 2, 3, 4, 6, 0, -.5, -1, -1.5, -2, -3, -4, -6], dtype=torch.float64)[torch.stack([c & 15, c >> 4], -1).long().flatten(1)]
+    c = torch.randint(0, 256, (N, Kd // 2), generator=g, dtype=torch.uint8, device=g.device)
+    values = torch.tensor([0, .5, 1, 1.5, 2, 3, 4, 6, 0, -.5, -1, -1.5, -2, -3, -4, -6], dtype=torch.float64, device=g.device)[torch.stack([c & 15, c >> 4], -1).long().flatten(1)]
     if kind == 3:
-        e = torch.randint(119, 123, (N, Kd // 32), generator=g, dtype=torch.uint8)
+        e = torch.randint(119, 123, (N, Kd // 32), generator=g, dtype=torch.uint8, device=g.device)
         return (*K().pack_mxfp4(c.cuda(), e.cuda()), 1, values * torch.exp2(e.double() - 127).repeat_interleave(32, 1))
-    s = (torch.rand(N, Kd // 16, generator=g) * 4 + 0.5).to(torch.float8_e4m3fn)
+    s = (torch.rand(N, Kd // 16, generator=g, device=g.device) * 4 + 0.5).to(torch.float8_e4m3fn)
     w = values * s.double().repeat_interleave(16, 1) * 0.25
     return (*K().pack_nvfp4(c.cuda(), s.cuda(), torch.tensor(0.25).cuda()), 1, w)
 
@@ -276,6 +276,8 @@ def test_prompt_attention_with_a_scale_of_zero_or_less(scale):
 def test_gemm_over_pairs_of_sms(T, N, Kd, epi, bias, f32):
     """Ragged tokens and features, rings shorter and longer than the k tiles, several tiles per pair of SMs, a last group of fewer token tiles; plain, gated
     and activated epilogues, fp32 and bf16 results. One rounding of an fp32 sum."""
+    from onecat_vllm.ops import _C
+    assert _C.gemm_route(T, N, Kd, 0, epi, f32, K()._sms(torch.device("cuda"))) == ("pair", 0)
     g = torch.Generator(device="cuda").manual_seed(T)
     x = torch.randn(T, Kd + 64, device="cuda", generator=g).bfloat16()[:, :Kd]
     w = (torch.randn(N, Kd, device="cuda", generator=g) * Kd ** -0.5).bfloat16()
@@ -299,20 +301,23 @@ def test_gemm_over_pairs_of_sms(T, N, Kd, epi, bias, f32):
 
 
 @pytest.mark.parametrize("kind", [1, 2, 3, 4])
-@pytest.mark.parametrize("T,N,Kd,gated", [(1100, 5120, 192, True), (2048, 1312, 704, False), (1024, 9984, 4224, False)])
-def test_packed_gemm_of_many_tokens(kind, T, N, Kd, gated):
-    """One slab of widened weights and several (5888 rows of 4224 k each), rows that end inside a tile, odd numbers of k tiles. Weights are rounded to bf16 where
-    they are widened; fp32 sums, one rounding at the end."""
-    g = torch.Generator().manual_seed(kind + T)
+@pytest.mark.parametrize("T,N,Kd,gated,slabs", [(1100, 5120, 192, True, 1), (2048, 1312, 704, False, 1), (1024, 13096, 8256, False, 2), (2048, 24096, 4224, True, 2), (1024, 9984, 4224, False, 0)])
+def test_packed_gemm_of_many_tokens(kind, T, N, Kd, gated, slabs):
+    """One slab of widened weights and two, whose second ends with the rows (bias, plain and gated columns, the slab reused while the product before
+    reads it), rows that end inside a tile, odd numbers of k tiles; none where tiles are the faster form. Weights are rounded to bf16 where they
+    are widened; fp32 sums, one rounding at the end."""
+    from onecat_vllm.ops import _C
+    assert _C.gemm_route(T, N, Kd, kind, 1 if gated else 0, False, K()._sms(torch.device("cuda"))) == (("widen", slabs) if slabs else ("tiles", 0))
+    g = torch.Generator(device="cuda").manual_seed(kind + T)
     tiles, sz, npad, gk, w = _packed(kind, N, Kd, g)
-    x = torch.randn(T, Kd, generator=g).bfloat16().cuda()
-    y = x.double() @ w.cuda().t()
+    x = torch.randn(T, Kd, generator=g, device="cuda").bfloat16()
+    y = x.double() @ w.t()
     bias = None
     if gated:
         pair = y.view(T, -1, 2, 16)
         want = (torch.nn.functional.silu(pair[:, :, 0]) * pair[:, :, 1]).reshape(T, -1)
     else:
-        bias = torch.randn(N, generator=g).bfloat16().cuda()
+        bias = torch.randn(N, generator=g, device="cuda").bfloat16()
         want = y + bias.double()
     out = torch.full((T + 1, want.shape[1] + 8), 7.0, dtype=torch.bfloat16, device="cuda")
     K()._gemm(x, None, tiles, sz, out[:T, : want.shape[1]], bias, N, N, want.shape[1], npad, 1 if gated else 0, gk, wkind=kind)
