@@ -89,11 +89,6 @@ __device__ __forceinline__ float head_gate(const AttnParams& p, size_t tok, int 
   return 1.f / (1.f + __expf(-__bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.gate)[tok * p.gate_st + head])));
 }
 
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 // tanh for soft caps in fp32: an odd polynomial (the series up to x^11, 3e-8 off at 0.4) near zero, (1 - e^-2x) / (1 + e^-2x) elsewhere
 constexpr float kTanhSmall = 0.4f;
 __device__ __forceinline__ float tanh_small(float x) {

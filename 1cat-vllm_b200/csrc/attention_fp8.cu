@@ -33,11 +33,6 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 // the bytes in bits 8-15 and 24-31 of t (the others may hold anything) as two bf16, times 2^-120
 __device__ __forceinline__ uint32_t place(uint32_t t, uint32_t mask, uint32_t sign) {
   uint32_t r;

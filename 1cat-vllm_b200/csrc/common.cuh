@@ -322,6 +322,51 @@ static inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 blo
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// ---- shared pieces of the kernels
+// 2^x, approximate
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// tanh form of GELU: 0.5 z (1 + tanh(u)) = z / (1 + 2^(-2u log2 e)), u = sqrt(2/pi) (z + 0.044715 z^3)
+__device__ __forceinline__ float gelu_tanh(float z) {
+  constexpr float c = -1.5957691216057308f * 1.4426950408889634f;
+  return z / (1.f + exp2f(z * fmaf(z * z, 0.044715f * c, c)));
+}
+
+// UMMA operand B, MN-major (its columns contiguous, as values lie in the paged caches): 64 columns x 8 keys form a 1024-byte swizzle atom; the next 8
+// keys are 1024 bytes on (stride byte offset), the next 64 columns `lbo_bytes` (leading byte offset).
+__device__ __forceinline__ uint64_t umma_desc_sw128_mn(uint32_t smem_addr, uint32_t lbo_bytes) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
+  d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+
+// Tensor map of bf16 [rows][cols], row pitch `ld` elements: boxes of {64 columns, box_rows rows}, 128-byte swizzle, zero fill. 0 when it was made.
+static inline int make_tmap_bf16(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
+  typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                    const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static EncodeTiledFn enc = nullptr;
+  if (!enc) {
+    void* ptr = nullptr;
+    cudaDriverEntryPointQueryResult qres;
+    cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres);
+    enc = reinterpret_cast<EncodeTiledFn>(ptr);
+  }
+  if (!enc) return -1;
+  cuuint64_t dims[2] = {cols, rows}, strides[1] = {ld * 2};
+  cuuint32_t box[2] = {64, box_rows}, estr[2] = {1, 1};
+  const CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : (int)r;
+}
+
 // Device address of this translation unit's status word on the current device (null when the runtime has none to give).
 static inline unsigned int* status_word_tu() {
   void* p = nullptr;

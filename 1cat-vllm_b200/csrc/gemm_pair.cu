@@ -28,11 +28,6 @@ constexpr int kSmem = kStages * kStage + 1024 + 1024;
 constexpr int kWidenTokens = 1024;                // see gemm_widen_takes
 constexpr int kGroup = 8;                         // token tiles of a group
 
-__device__ __forceinline__ float gelu_tanh(float z) {
-  constexpr float c = -1.5957691216057308f * 1.4426950408889634f;
-  return z / (1.f + exp2f(z * fmaf(z * z, 0.044715f * c, c)));
-}
-
 // TMA copy into this CTA's shared memory, counted by a barrier of either CTA of the pair (a shared::cluster address)
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* tm, int x, int y, uint32_t bar) {
   asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -254,25 +249,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// bf16 [rows][cols], row pitch ld elements -> boxes of {64 columns, 128 rows}, 128-byte swizzle, zero fill
-int make_tmap(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t cols, uint64_t ld) {
-  static EncodeTiledFn enc = nullptr;
-  if (!enc) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres);
-    enc = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
-  if (!enc) return -1;
-  cuuint64_t dims[2] = {cols, rows}, strides[1] = {ld * 2};
-  cuuint32_t box[2] = {64, 128}, estr[2] = {1, 1};
-  return enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -2;
-}
-
 }  // namespace
 
 // Takes more than 128 tokens (fewer leave half of a tile empty) with tiles for at least half of the pairs; below that the split k ranges of
@@ -287,8 +263,8 @@ int gemm_pair_launch(const GemmParams& p_in, const void* x, int ldx, const void*
   GemmParams p = p_in;
   if (p.K % 64 || p.K <= 0) return -1;
   CUtensorMap tmX, tmW;
-  if (make_tmap(&tmX, x, (uint64_t)p.T, (uint64_t)p.K, (uint64_t)ldx)) return -2;
-  if (make_tmap(&tmW, w, (uint64_t)p.n_rows, (uint64_t)p.K, (uint64_t)ldw)) return -3;
+  if (make_tmap_bf16(&tmX, x, (uint64_t)p.T, (uint64_t)p.K, (uint64_t)ldx, 128)) return -2;
+  if (make_tmap_bf16(&tmW, w, (uint64_t)p.n_rows, (uint64_t)p.K, (uint64_t)ldw, 128)) return -3;
   p.num_t_tiles = (p.T + kTok - 1) / kTok;
   p.num_n_tiles = (p.n_rows + kFeat - 1) / kFeat;
   p.vec_ok = p.out != nullptr && (p.ldo % 8 == 0) && ((uintptr_t)p.out & 15) == 0;

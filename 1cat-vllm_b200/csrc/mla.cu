@@ -36,12 +36,6 @@ __device__ __forceinline__ uint32_t pk(float lo, float hi) {
 __device__ __forceinline__ uint32_t koff(int row, int chunk, int pitch) { return (uint32_t)(row * pitch * 2 + (((chunk & ~7) | ((chunk ^ row) & 7)) << 4)); }
 __device__ __forceinline__ float rounded(float v) { return __bfloat162float(__float2bfloat16(v)); }
 
-__device__ __forceinline__ float ex2(float x) {   // approximate instruction: the softmax of the bf16 kernels
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 template <typename E> __device__ __forceinline__ float ldf(const E* p);
 template <> __device__ __forceinline__ float ldf<float>(const float* p) { return *p; }
 template <> __device__ __forceinline__ float ldf<__nv_bfloat16>(const __nv_bfloat16* p) { return __bfloat162float(*p); }

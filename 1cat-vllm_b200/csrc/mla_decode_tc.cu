@@ -38,22 +38,8 @@ constexpr int kThreads = 192;
 constexpr uint32_t kColO = 0, kColS = 256, kColQ = 384;          // TMEM columns: O | S0 | S1 | Q of group B
 constexpr float kLazy = 8.f;                 // growth of a maximum (log2) that is left in the weights
 
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // V as operand B, MN-major: 64 columns x 8 keys form a 1024-byte swizzle atom; the next 8 keys are 1024 bytes on, the next 64 columns a chunk on
-__device__ __forceinline__ uint64_t desc_v(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)((kKChunk >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
+__device__ __forceinline__ uint64_t desc_v(uint32_t smem_addr) { return umma_desc_sw128_mn(smem_addr, kKChunk); }
 
 // element j of a rotated row (see mla.cu)
 __device__ __forceinline__ float rotated(const __nv_bfloat16* x, int j, int n, const float* cs, int interleaved) {
@@ -405,25 +391,6 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// bf16 [rows][cols] -> boxes of {64 columns, box_rows rows}, 128-byte swizzle, zero fill
-int make_tmap(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
-  static EncodeTiledFn enc = nullptr;
-  if (!enc) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres);
-    enc = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
-  if (!enc) return -1;
-  cuuint64_t dims[2] = {cols, rows}, strides[1] = {cols * 2};
-  cuuint32_t box[2] = {64, box_rows}, estr[2] = {1, 1};
-  return enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -2;
-}
-
 }  // namespace
 
 // What this kernel can run: DeepSeek's latent width, weights in one term, pages of whole 16-key pieces (a TMA box) and positive scales
@@ -437,8 +404,8 @@ bool mla_decode_tc_takes(int kv_lora, int rope_pad, int bs, int fine, float scal
 int mla_decode_tc_launch(const MlaParams& p, cudaStream_t st) {
   if (((uintptr_t)p.q_abs & 15) || ((uintptr_t)p.cache & 15) || ((uintptr_t)p.out & 15) || p.num_blocks <= 0) return -1;
   CUtensorMap tmQ, tmK;
-  if (make_tmap(&tmQ, p.q_abs, (uint64_t)p.T * p.H, DV, TM)) return -2;
-  if (make_tmap(&tmK, p.cache, (uint64_t)p.num_blocks * p.bs, (uint64_t)(DV + p.rope_pad), 16)) return -3;
+  if (make_tmap_bf16(&tmQ, p.q_abs, (uint64_t)p.T * p.H, DV, DV, TM)) return -2;
+  if (make_tmap_bf16(&tmK, p.cache, (uint64_t)p.num_blocks * p.bs, (uint64_t)(DV + p.rope_pad), (uint64_t)(DV + p.rope_pad), 16)) return -3;
   static bool configured_dev[kMaxDevices] = {};
   bool& configured = configured_dev[current_device_slot()];  // the limit is an attribute of (kernel, device)
   if (!configured) {

@@ -25,22 +25,8 @@ constexpr int kStages = 2;
 constexpr int kThreads = 320;
 constexpr uint32_t kColS = 0, kColO = 256;   // TMEM columns: S0 | S1 | O_tile
 
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // MN-major operand B: 64 columns x 8 rows form a 1024-byte swizzle atom; the next 8 rows (k) are 1024 bytes on, the next 64 columns a chunk on.
-__device__ __forceinline__ uint64_t desc_mn(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)((kChunk >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
+__device__ __forceinline__ uint64_t desc_mn(uint32_t smem_addr) { return umma_desc_sw128_mn(smem_addr, kChunk); }
 
 template <int QC, int VC>
 constexpr int smem_bytes() { return QC * kChunk + kStages * (QC + VC) * kChunk + 1024 + 2 * 2 * TQ * 4; }
@@ -391,39 +377,13 @@ __global__ void __launch_bounds__(256) mla_query_kernel(const MlaPrefillParams p
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn get_encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres);
-    fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
-  return fn;
-}
-
-// bf16 [rows][cols] -> boxes of {64 columns, 128 rows}, 128-byte swizzle, zero fill
-int make_tmap(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t cols) {
-  EncodeTiledFn enc = get_encode_fn();
-  if (!enc) return -1;
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {cols * 2};
-  cuuint32_t box[2] = {64, 128};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : (int)r;
-}
-
 template <int QC, int VC, bool FINE>
 int go(const MlaPrefillParams& p, cudaStream_t st) {
+  auto tmap = [](CUtensorMap* tm, const void* base, uint64_t rows, uint64_t cols) { return make_tmap_bf16(tm, base, rows, cols, cols, 128); };
   CUtensorMap tmQ, tmKV, tmR;
-  if (make_tmap(&tmQ, p.q_out, (uint64_t)p.T, (uint64_t)p.H * QC * 64)) return -2;
-  if (make_tmap(&tmKV, p.kv, (uint64_t)p.rows, (uint64_t)p.H * (p.NC + VC) * 64)) return -3;
-  if (make_tmap(&tmR, p.rot, (uint64_t)p.rows, (uint64_t)p.RC * 64)) return -3;
+  if (tmap(&tmQ, p.q_out, (uint64_t)p.T, (uint64_t)p.H * QC * 64)) return -2;
+  if (tmap(&tmKV, p.kv, (uint64_t)p.rows, (uint64_t)p.H * (p.NC + VC) * 64)) return -3;
+  if (tmap(&tmR, p.rot, (uint64_t)p.rows, (uint64_t)p.RC * 64)) return -3;
   constexpr int smem = smem_bytes<QC, VC>() + 1024;
   static bool configured_dev[kMaxDevices] = {};
   bool& configured = configured_dev[current_device_slot()];

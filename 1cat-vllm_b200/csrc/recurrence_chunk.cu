@@ -24,11 +24,6 @@ constexpr float kLog2e = 1.4426950408889634f;
 
 __device__ __forceinline__ float softplus(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 // 2^x for exponents that are not positive (2 ulp)
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 __device__ __forceinline__ float bf(const __nv_bfloat16 v) { return __bfloat162float(v); }
 
 // two neighbouring outputs, as far as `left` columns go

@@ -24,11 +24,6 @@ constexpr int kSlots = 10, kSlot = kChunk, kVChunk = 32 * 128, kThreads = 576;  
 constexpr uint32_t kColS = 0, kColO = 256;
 constexpr float kLog2e = 1.4426950408889634f, kSlack = 8.f, kNear = 1.f / 16.f;
 
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 __device__ __forceinline__ float lg2(float x) {
   float y;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -64,15 +59,7 @@ __device__ __forceinline__ f2 add2(f2 a, f2 b) {
 }
 
 // MN-major operand B: 64 columns x 8 keys form a 1024-byte swizzle atom; the next 8 keys are 1024 bytes on, the next 64 columns 32 keys on.
-__device__ __forceinline__ uint64_t desc_mn(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)((kVChunk >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
+__device__ __forceinline__ uint64_t desc_mn(uint32_t smem_addr) { return umma_desc_sw128_mn(smem_addr, kVChunk); }
 
 // the 128 threads of a lane quarter (four warps): barrier, and barrier with a vote
 __device__ __forceinline__ void quarter_sync(int q) { asm volatile("bar.sync %0, 128;" ::"r"(q + 1) : "memory"); }
@@ -450,30 +437,11 @@ talk_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// bf16 [rows][cols], contiguous -> boxes of {64 columns, box_rows rows}, 128-byte swizzle, zero fill
-int make_tmap(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
-  static EncodeTiledFn enc = nullptr;
-  if (!enc) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres);
-    enc = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
-  if (!enc) return -1;
-  cuuint64_t dims[2] = {cols, rows}, strides[1] = {cols * 2};
-  cuuint32_t box[2] = {64, box_rows}, estr[2] = {1, 1};
-  return enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -1;
-}
-
 template <int NC>
 int go(TalkTcParams p, int tiles, int segment, long long num_blocks, cudaStream_t st) {
   CUtensorMap tmQ, tmK;
-  if (make_tmap(&tmQ, p.t.q, (uint64_t)p.t.T, (uint64_t)p.t.H * NC * 64, TQ)) return -2;
-  if (make_tmap(&tmK, p.t.pages, (uint64_t)num_blocks * p.t.G * p.t.bs, NC * 64, 16)) return -3;
+  if (make_tmap_bf16(&tmQ, p.t.q, (uint64_t)p.t.T, (uint64_t)p.t.H * NC * 64, (uint64_t)p.t.H * NC * 64, TQ)) return -2;
+  if (make_tmap_bf16(&tmK, p.t.pages, (uint64_t)num_blocks * p.t.G * p.t.bs, NC * 64, NC * 64, 16)) return -3;
   constexpr int smem = smem_bytes<NC>() + 1024;
   static bool configured_dev[kMaxDevices] = {};
   bool& configured = configured_dev[current_device_slot()];
