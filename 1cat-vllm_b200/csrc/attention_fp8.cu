@@ -11,9 +11,9 @@
 //     is one 16-byte chunk of a key row.
 //   * P V: the eight columns of a step may be any dimensions, so lane group g takes chunk g of a value row, and column n of step j is dimension
 //     16 n + j; a pair of keys is two bytes of neighbouring rows, put together by one byte permutation.
-// Bound by memory, then by those integer instructions (57 us of ALU time for 8 requests x 32768 keys x 8 heads of 128, 78 us of
-// memory). Measured with the merge of the splits, against the kernel that widened tiles into shared memory: 8 requests x 32768 keys x 8 heads of
-// 128 144 us for 219, 4 heads of 256 136 for 279; 64 requests x 1152 keys 55 for 80; one request x 32000 keys 38 for 52.
+// 8 requests x 32768 keys x 8 heads of 128: those integer instructions keep the ALU pipe 62 % busy with twelve warps an SM, memory 46 %; latencies are the
+// rest. Measured with the merge of the splits, against the kernel that widened tiles into shared memory (us): that case 148 / 219, 4 heads of 256 136 / 279; 64
+// requests x 1152 keys 56 / 80; one request x 32000 keys 38 / 52.
 // (reference: csrc/attention/paged_attention_v2.cu with fp8 caches; v1/attention/backends/flash_attn.py)
 #include "common.cuh"
 #include "kernels.h"

@@ -10,8 +10,8 @@
 // accumulator is at rest; a row whose maximum has grown by more than 2^8 since its reference rescales it then (smaller growth stays in
 // the weights: their reference cancels in the division). Query tiles go out longest first, all heads of a tile together.
 // Bound: 1024 tensor cycles per 128 x 128 tile, and as many for its 16384 exponentials at 16 a cycle. Measured: 8192
-// tokens x 40 heads 650 us (1.06 PFLOP/s; one tile of 128 rows per CTA with its results summed in registers took 1520); a prompt of 1024 tokens
-// 47 us for 63. Handing the weights over in two halves, so that the value product starts earlier, was no faster.
+// tokens x 40 heads 657 us (1.05 PFLOP/s, tensor pipe and exponentials 49 % busy each; one tile of 128 rows per CTA with its results summed in registers takes 1535); a prompt of
+// 1024 tokens 33 us for 55. Handing the weights over in two halves, so that the value product starts earlier, was no faster.
 // Roles: warp 0 = TMA producer (the 16 page loads of a K or V tile are issued by 16 lanes at once), warp 1 = MMA issue, warps 2-5 and 6-9 =
 // softmax and epilogue of the two query tiles.
 // Every wait is bounded; on expiry the CTA raises the status word and tears down (see common.cuh).

@@ -171,9 +171,8 @@ __global__ void silu_and_mul_kernel(const __nv_bfloat16* __restrict__ x, __nv_bf
 
 // The same in 16-byte accesses: a group of D / 8 lanes owns a head, a lane eight neighbouring elements of it; the other element of each rotary
 // pair comes from the lane half a rotary width away. A group takes HU heads of a token with their loads in flight together and the token's
-// cosines and sines read once. Bound by memory: a prompt's q, k and v once in and once out. Two-byte accesses with a warp per head
-// (rope_cache_kernel below) reached 0.8 TB/s at 8192 tokens x 56 heads of 128 (295 us); this one
-// takes 80 us (2.9 TB/s); at 64 tokens 8 us for 10.
+// cosines and sines read once. Bound by instruction issue (conversions and shuffles: 68 % of the slots, memory at 32 %). 8192 tokens x 56 heads of 128: 78 us,
+// where two-byte accesses with a warp per head (rope_cache_kernel below) take 222; 1087 tokens 20.5 / 37, 64 tokens 8 / 10.
 template <int D, int HU>
 __global__ void __launch_bounds__(256) rope_cache_vec_kernel(const RopeCacheParams p) {
   constexpr int LPH = D / 8;                     // lanes of a head

@@ -11,8 +11,8 @@
 // Two accumulators of 256 columns: the epilogue of a tile overlaps the products of the next. Tiles go out in groups of eight token tiles, feature
 // tiles outside, so that what is in flight at a time shares both operands in L2.
 // Every wait is bounded (see common.cuh); when a role gives up in one CTA, the other CTA's waits run out too, and both meet at the end.
-// Measured against the single-CTA tiles of gemm_sm100.cu: 8192 x 34816 x 5120 1781 us for 2343 (1.64 PFLOP/s), 1024 x 34816 x 5120 234 for 301,
-// 8192 x 5120 x 5120 277 for 356, 300 x 16384 x 5120 83 for 114.
+// Bound by the tensor pipe (95 % busy), in long products by power. Measured against the single-CTA tiles of gemm_sm100.cu: 8192 x 34816 x 5120 1781 to
+// 1858 us (1.57 to 1.64 PFLOP/s) for 2343, 1024 x 34816 x 5120 235 for 301, 8192 x 5120 x 5120 277 for 356, 300 x 16384 x 5120 83 for 114.
 // (reference: cuBLAS for unquantised layers)
 #include "common.cuh"
 #include "gemm_sm100.h"

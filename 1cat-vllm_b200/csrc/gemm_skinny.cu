@@ -12,8 +12,8 @@
 //     more than the order of fp32 sums.
 // The warps of a CTA take the units of its 32 rows in turn and meet once, for the sum over k and the epilogue.
 // Packed bf16 arithmetic comes next: a scheduler takes about four cycles for one such instruction, and a 16 x 64 block of int4 has 32 of them
-// (and 43 on the integer pipe). Measured on 34816 x 5120 int4 rows and 4 tokens: 45 us where the tcgen05 path takes 54 (2 TB/s); 2048 x 1024: 8
-// where it takes 16.
+// (and 43 on the integer pipe, 48 % busy, issue slots 55 %). Measured on 34816 x 5120 int4 rows and 4 tokens: 46 us where the tcgen05 path takes 54 (2
+// TB/s); 2048 x 1024: 8 where it takes 15.
 // (reference: the decode GEMMs of csrc/sm70_turbomind; csrc/quantization/gptq_marlin)
 #include "common.cuh"
 #include "gemm_sm100.h"

@@ -16,9 +16,10 @@
 // weights' reference cancels in the division), by the softmax warps, which then wait for the value products issued so far.
 // Roles: warp 0 TMA producer, warp 1 MMA issue, warps 2-5 queries, softmax and epilogue. Every wait is bounded (see common.cuh).
 //
-// Bound: 8.7 M products per key tile and CTA, about 2250 cycles at 32 cycles per 128 x 64 x 16 product and 48 where operand A comes from
-// shared memory (its reads then need 6 KB per instruction at 128 bytes a cycle). Measured (kernel
-// and merge): 32 requests x 4096 keys x 128 heads 97 us where the mma.sync kernel takes 706, of which 23 us are the cache's 150 MB from memory.
+// Bound: 128 x 64 x (576 + 256) = 6.8 M products per key tile and CTA, about 1980 cycles at 32 cycles per 128 x 64 x 16 product and 48 where operand
+// A comes from shared memory (its reads then need 6 KB per instruction at 128 bytes a cycle). A tile takes about 4900: one softmax warp per scheduler and
+// the tensor pipe (37 % busy) hand scores and weights to each other. Measured (kernel and merge): 32 requests x 4096 keys x 128 heads 99 us, two splits on
+// 128 of 148 SMs, where the mma.sync kernel takes 730; the cache's 150 MB alone are 23 us of memory.
 // (reference: csrc/attention/mla/sm100_cutlass_mla_kernel.cu)
 #include "common.cuh"
 #include "kernels.h"
