@@ -111,7 +111,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         // Rows of long k lie far apart, and a k tile at a time is 128 bytes from each: there the group's first pair brings the weights of eight k
         // tiles at a time to L2 (17408 k, 5120 features: 512 tokens 155 -> 130 us, 4096 685 -> 544; at 5120 k it costs 8 %, and at 8192
         // tokens the other operand sets the pace).
-        const bool lead = p.K >= 8192 && tt_all <= 2 * kGroup && tt % kGroup == 0;
+        const bool lead = p.K >= 8192 && tt_all <= 2 * kGroup && tt % kGroup == 0 && y1 < p.n_rows;   // a half past the rows has nothing to bring
         for (int kt = 0; kt < ktiles; ++kt) {
           if (lead && kt % 8 == 0) {
             const int k1 = min(kt + 16, ktiles);

@@ -272,9 +272,11 @@ def test_prompt_attention_with_a_scale_of_zero_or_less(scale):
 
 
 @pytest.mark.parametrize("T,N,Kd,epi,bias,f32", [(256, 9472, 64, 0, False, False), (300, 5120, 640, 0, True, False), (2500, 1000, 1088, 0, True, True), (129, 9600, 128, 1, False, False),
-                                                 (1030, 2112, 448, 3, False, False), (515, 3336, 192, 2, True, False), (9000, 520, 256, 0, False, False)])
+                                                 (1030, 2112, 448, 3, False, False), (515, 3336, 192, 2, True, False), (9000, 520, 256, 0, False, False),
+                                                     (2500, 1096, 8256, 0, True, True), (700, 3300, 8192, 0, False, False)])
 def test_gemm_over_pairs_of_sms(T, N, Kd, epi, bias, f32):
-    """Ragged tokens and features, rings shorter and longer than the k tiles, several tiles per pair of SMs, a last group of fewer token tiles; plain, gated
+    """Ragged tokens and features, rings shorter and longer than the k tiles, several tiles per pair of SMs, a last group of fewer token tiles, long k (weights are
+    brought to L2 ahead; halves of tiles past the rows); plain, gated
     and activated epilogues, fp32 and bf16 results. One rounding of an fp32 sum."""
     from onecat_vllm.ops import _C
     assert _C.gemm_route(T, N, Kd, 0, epi, f32, K()._sms(torch.device("cuda"))) == ("pair", 0)
