@@ -637,7 +637,10 @@ def paged_attention(q, kv_cache, md, scale, out=None, lse=None, window=0, softca
     if tiles:
         if (D == 128 and q.stride(1) == D and _ATTN_PREFILL_TC and scale > 0 and not window and not softcap and sinks is None and not extended
                 and kv_cache.dtype == torch.bfloat16):
-            pairs, tiles_tc = prompt_tiles(md.query_lens_cpu, md.seq_lens_cpu, short, Hq, _sms(q.device))
+            pieces = md.__dict__.setdefault("_prompt_tiles", {})   # of this step: its layers share them
+            if (short, Hq) not in pieces:
+                pieces[short, Hq] = prompt_tiles(md.query_lens_cpu, md.seq_lens_cpu, short, Hq, _sms(q.device))
+            pairs, tiles_tc = pieces[short, Hq]
             _C.paged_attention(q, kv_cache, out, lse, md.query_start_loc, md.seq_lens, md.block_table, scale, 2 if pairs else 4, tiles_tc, 1,
                                md.max_query_len, short, None, None, 0, 0.0, None, 1.0, 1.0)
         else:
@@ -912,8 +915,11 @@ def mla_decode(q_abs, q_pe, latent_cache, md, scale, lora, cos_sin=None, interle
         if static and plan is not None and plan[0][0] == "mla":
             splits, wide = plan[1][2]  # captured decode graph: both are part of the graph's key
         else:
-            wide = mla_decode_wide(lora, latent_cache.shape[-1] - lora, latent_cache.shape[1], fine, scale)
-            splits, wide = plan_mla(H, lora, ql, sl, _sms(q_abs.device), wide)
+            plans, key = md.__dict__.setdefault("_mla_plans", {}), (H, lora, latent_cache.shape[1:], fine, scale, skip_min_len)
+            if key not in plans:   # of this step: its layers share them
+                wide = mla_decode_wide(lora, latent_cache.shape[-1] - lora, latent_cache.shape[1], fine, scale)
+                plans[key] = plan_mla(H, lora, ql, sl, _sms(q_abs.device), wide)
+            splits, wide = plans[key]
         if splits > 1:
             w = workspace(q_abs.device)
             ws_o, ws_ml = (w.attn_static if static else w.attn)(splits * T * H * lora, splits * T * H * 4)   # a reference and a sum for each half of the columns
